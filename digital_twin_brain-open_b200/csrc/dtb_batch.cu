@@ -30,12 +30,11 @@ Batch::~Batch() {
     if (stream) cudaStreamSynchronize(stream);
     if (graph) cudaGraphExecDestroy(graph);
     for (void* p : {static_cast<void*>(d_views), static_cast<void*>(d_prefix), static_cast<void*>(list),
-                    static_cast<void*>(list_count), static_cast<void*>(list_ticket), static_cast<void*>(local_scratch),
+                    static_cast<void*>(list_count), static_cast<void*>(list_published), static_cast<void*>(local_scratch),
                     static_cast<void*>(tile_net)})
         if (p) cudaFree(p);
-    for (cudaEvent_t e : {ev0, ev1, tev[0], tev[1], ev_fork, ev_join})
+    for (cudaEvent_t e : {ev0, ev1, tev[0], tev[1]})
         if (e) cudaEventDestroy(e);
-    if (aux) cudaStreamDestroy(aux);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -45,9 +44,6 @@ int Batch::create(Engine* const* engines, uint32_t n) {
     DTB_CU(cudaEventCreate(&ev1));
     DTB_CU(cudaEventCreate(&tev[0]));
     DTB_CU(cudaEventCreate(&tev[1]));
-    DTB_CU(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
-    DTB_CU(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    DTB_CU(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     return set_members(engines, n);
 }
 
@@ -107,17 +103,15 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
     if (windows > cap_windows) {
         if (local_scratch) cudaFree(local_scratch);
         local_scratch = nullptr;
-        DTB_CU(cudaMalloc(reinterpret_cast<void**>(&local_scratch), sizeof(uint32_t) * (2ull * windows + 3)));
+        DTB_CU(cudaMalloc(reinterpret_cast<void**>(&local_scratch), sizeof(uint32_t) * local_scratch_words(windows)));
         cap_windows = windows;
     }
-    // the prep kernel's block ticket sits after this membership's tables: start it at zero
-    if (local_scratch) DTB_CU(cudaMemsetAsync(local_scratch, 0, sizeof(uint32_t) * (2ull * cap_windows + 3), stream));
     if (!list_count) {
         DTB_CU(cudaMalloc(reinterpret_cast<void**>(&list_count), sizeof(uint32_t)));
-        DTB_CU(cudaMalloc(reinterpret_cast<void**>(&list_ticket), sizeof(uint32_t)));
+        DTB_CU(cudaMalloc(reinterpret_cast<void**>(&list_published), 2 * sizeof(uint32_t)));
     }
     DTB_CU(cudaMemsetAsync(list_count, 0, sizeof(uint32_t), stream));
-    DTB_CU(cudaMemsetAsync(list_ticket, 0, sizeof(uint32_t), stream));
+    DTB_CU(cudaMemsetAsync(list_published, 0, 2 * sizeof(uint32_t), stream));
     DTB_CU(cudaMemcpyAsync(d_prefix, pre.data(), sizeof(uint32_t) * pre.size(), cudaMemcpyHostToDevice, stream));
     lb.nets = d_views;
     lb.lif_prefix = d_prefix;
@@ -129,15 +123,14 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
     lb.push_ctas = static_cast<uint32_t>(sm_count) * 8u;
     lb.lif_ctas = static_cast<uint32_t>(sm_count) * m[0]->lif_ctas_per_sm;
     lb.lif_chunk = n > 1 ? kBatchLifChunk : 1u;
-    lb.spikes = SpikeList{list, list_count, list_ticket, static_cast<uint32_t>(total)};
+    lb.spikes = SpikeList{list, list_count, list_published, static_cast<uint32_t>(total)};
     lb.tile_net = tile_net;
-    lb.win_prefix = d_prefix + 3 * (n + 1);
-    lb.windows_total = windows;
-    lb.local_scratch = local_scratch;
+    uint64_t edges = 0;
+    for (const Engine* e : m) edges += e->n_edges;
+    dense_min = dense_min_spikes(edges, total);
+    windows_total = windows;
+    lb.local = LocalPlan{d_prefix + 3 * (n + 1), windows, dense_min, 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch};
     lb.sm_count = static_cast<uint32_t>(sm_count);
-    lb.aux = aux;
-    lb.ev_fork = ev_fork;
-    lb.ev_join = ev_join;
     if (graph) {
         cudaGraphExecDestroy(graph);
         graph = nullptr;
@@ -223,6 +216,8 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
             push_tuned[acc] = it != tuned_by_size[acc].end();
             if (push_tuned[acc]) push_cfg = it->second;
         }
+        lb.local.dense_min = window_always ? 1u : dense_min;
+        lb.local.always = window_always ? 1u : 0u;
         DTB_CU(push_prepare(acc, wt, push_cfg, sm_count, &push_ctas));
         if (autotune && !push_tuned[acc]) {
             const uint64_t settle = 300;
@@ -251,11 +246,16 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
         // starts a run folds nothing into J on its first step, and the last chunk of an
         // exact or fixed run ends by folding the sums into J, so both are in the key.
         const bool last_chunk = done + rows == rq.iters;
-        const bool graphable = use_graph && !pull && !(tune_at >= done && tune_at < done + rows);
+        const bool tune_here = tune_at >= done && tune_at < done + rows;
+        const bool graphable = use_graph && !pull && !tune_here;
+        // the LIF kernel prepares the windows' work units when this chunk's pushes (or the tuner's) read them
+        lb.local.flush_reds = acc == ACC_FIXED ? 2u : 1u;
+        lb.local.windows = acc != ACC_EXACT && (push_cfg.kind == PUSH_LOCAL || tune_here) ? windows_total : 0u;
         bool replay = false;
         if (graphable) {
             const uint64_t key[9] = {rows, kflags, static_cast<uint64_t>(pm),
-                                     static_cast<uint64_t>(push_cfg.kind) * 100000 + push_cfg.param * 100 + push_cfg.lpr,
+                                     static_cast<uint64_t>(push_cfg.kind) * 100000 + push_cfg.param * 100 + push_cfg.lpr +
+                                         (static_cast<uint64_t>(lb.local.dense_min) << 32),
                                      push_ctas, rq.syn_mode, done == 0, last_chunk, 1};
             if (graph && std::memcmp(key, graph_key, sizeof(key)) == 0) {
                 replay = true;
@@ -291,7 +291,7 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
         if (replay) {
             DTB_CU(cudaGraphLaunch(graph, stream));
             ++graph_launches;
-            launches += (2 + push_extra_launches(lb, acc, push_cfg) + (isyn_any ? 1u : 0u)) * rows +
+            launches += (2 + (isyn_any ? 1u : 0u)) * rows +
                         (last_chunk && acc != ACC_FLOAT ? 1u : 0u);
         } else {
             for (uint32_t s = 0; s < rows; ++s) {
@@ -313,7 +313,7 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
                     }
                     DTB_TRY(tune_push_views(lb, v, acc, wt, sm_count, stream, tev, tune));
                     if (tune.tuned) {
-                        push_cfg = tune.best;
+                        if (!tune.report.empty()) push_cfg = tune.best;
                         push_tuned[acc] = true;
                         tuned_by_size[acc][size_class] = push_cfg;
                         tune.reset();
@@ -323,7 +323,7 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
                     }
                 }
                 DTB_CU(launch_push(lb, acc, wt, push_cfg, push_ctas, stream));
-                launches += 2 + push_extra_launches(lb, acc, push_cfg);
+                launches += 2;
                 if (isyn_any) {
                     DTB_CU(launch_stat_isyn(lb, acc, sm_count, stream));
                     ++launches;
@@ -416,6 +416,7 @@ int32_t dtb_batch_set_push_variant(void* batch, int32_t kind, int32_t param) {
     Batch* b = static_cast<Batch*>(batch);
     if (kind < 0) {
         b->autotune = true;
+        b->window_always = false;
         for (int a = 0; a < 3; ++a) {
             b->push_tuned[a] = false;
             b->tuned_by_size[a].clear();
@@ -427,6 +428,7 @@ int32_t dtb_batch_set_push_variant(void* batch, int32_t kind, int32_t param) {
     if (!dtb::push_cfg_from_abi(kind, param, cfg)) return dtb::fail(DTB_INVALID_PARAMETER, "unknown push variant");
     b->push_cfg = cfg;
     b->autotune = false;
+    b->window_always = true;
     return DTB_OK;
 }
 

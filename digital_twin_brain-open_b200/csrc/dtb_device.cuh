@@ -152,6 +152,8 @@ struct NetView {
     const uint32_t* woff;          // row j of population a: woff[rb(a) + (j - pop_off[a]) * (k_a + 1) + k]
     const uint4* pop_loc;          // [n_pops] {k_a, window width, rb(a) low word, rb(a) high word}
     const uint4* win_tab;          // [n_windows] {population, first neuron, end neuron, window index | s << 16}
+    uint32_t* pop_live;            // [n_pops] spiking rows of the step being stepped, per population
+    const uint2* pop_win;          // [n_pops] {first window, spiking rows from which the windows pay}
     uint32_t n_windows;
     // Fixed-point push (DTB_SYN_PUSH_FIXED): one step's input to neuron i as two
     // pairs of unsigned 32-bit sums in units of 2^-fix_shift, receptor pair k in
@@ -166,8 +168,8 @@ struct NetView {
 // Batch-wide spike list written by the LIF kernel and consumed by the push kernel.
 struct SpikeList {
     uint32_t* list;                // virtual neuron ids: vbase[net] + neuron
-    uint32_t* count;
-    uint32_t* ticket;              // last-CTA counter of the push kernel
+    uint32_t* count;               // entries so far in the step being stepped
+    uint32_t* published;           // [0] the finished step's list length, read by the push; [1] finished networks of the launch
     uint32_t capacity;
 };
 

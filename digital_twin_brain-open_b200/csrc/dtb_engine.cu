@@ -29,7 +29,6 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 __global__ void set_u64_kernel(unsigned long long* p, unsigned long long v) { *p = v; }
-__global__ void set_u32_kernel(uint32_t* p, uint32_t v) { *p = v; }
 
 static constexpr size_t kCsrPadWords = 16;   // 64 bytes after every CSR array
 static constexpr size_t kCsrPadBytes = 64;
@@ -56,9 +55,6 @@ Engine::~Engine() {
     if (tune_ev[1]) cudaEventDestroy(tune_ev[1]);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (aux) cudaStreamDestroy(aux);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -90,9 +86,6 @@ int Engine::init_common(const dtb_options& opt, uint32_t n_neurons) {
     DTB_CU(cudaGetDevice(&device));
     DTB_CU(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
     DTB_CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    DTB_CU(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
-    DTB_CU(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    DTB_CU(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     DTB_CU(cudaEventCreate(&ev0));
     DTB_CU(cudaEventCreate(&ev1));
     dt = opt.dt;
@@ -226,6 +219,8 @@ int Engine::refresh_view() {
     v.woff = woff;
     v.pop_loc = pop_loc;
     v.win_tab = win_tab;
+    v.pop_win = pop_win;
+    v.pop_live = pop_live;
     v.n_windows = n_windows;
     v.dJf = dJf;
     v.fix_shift = fix_shift;
@@ -249,14 +244,11 @@ LaunchBatch Engine::single_batch() const {
     b.push_ctas = static_cast<uint32_t>(sm_count) * 8u;
     b.lif_ctas = static_cast<uint32_t>(sm_count) * lif_ctas_per_sm;
     b.lif_chunk = 1;
-    b.spikes = SpikeList{list, list_count, list_ticket, n_pad};
-    b.win_prefix = prefix_dev + 6;
-    b.windows_total = n_windows;
-    b.local_scratch = local_scratch;
+    b.spikes = SpikeList{list, list_count, list_published, n_pad};
+    // a chosen window form takes the windows in every step, the tuner's choice in busy steps only
+    b.local = LocalPlan{prefix_dev + 6, n_windows, window_always ? 1u : dense_min_spikes(n_edges, n),
+                        window_always ? 1u : 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch};
     b.sm_count = static_cast<uint32_t>(sm_count);
-    b.aux = aux;
-    b.ev_fork = ev_fork;
-    b.ev_join = ev_join;
     return b;
 }
 
@@ -300,6 +292,7 @@ uint32_t fixed_shift_for(uint64_t max_in_degree, double max_w, bool negative) {
 // resolution of 2^-kLocalMinShift or finer; other populations stay with the
 // scattered push.
 constexpr double kLocalMinSpan = 32.0;
+constexpr double kFlushEvents = 4.0, kUnitEvents = 8192.0;   // events per window neuron, and per window, that pay for its sums
 constexpr int kLocalMinShift = 16;
 constexpr int kLocalMaxShift = 60;
 
@@ -327,6 +320,7 @@ int Engine::build_local_tables() {
     if (unsorted) return DTB_OK;
     std::vector<uint4> loc(P, make_uint4(0, 0, 0, 0));
     std::vector<uint4> wins;
+    std::vector<uint2> first(P, make_uint2(0, 0));
     unsigned long long rb = 0;
     for (uint32_t a = 0; a < P; ++a) {
         const uint32_t size = pop_off[a + 1] - pop_off[a];
@@ -348,6 +342,10 @@ int Engine::build_local_tables() {
         while (sh >= kLocalMinShift && static_cast<double>(mw) * deg * std::ldexp(1.0, sh) >= room) --sh;
         if (sh < kLocalMinShift) continue;
         const uint32_t width = (size + k - 1) / k;
+        // a window costs a reduction per neuron to flush, and a unit's start-up: its events must outnumber them
+        const double own = static_cast<double>(total) / size;
+        first[a] = make_uint2(static_cast<uint32_t>(wins.size()),
+                              static_cast<uint32_t>(std::ceil(k * (kFlushEvents * width + kUnitEvents) / own)));
         loc[a] = make_uint4(k, width, static_cast<uint32_t>(rb), static_cast<uint32_t>(rb >> 32));
         for (uint32_t w = 0; w < k; ++w) {
             const uint32_t lo = std::min<uint64_t>(pop_off[a] + static_cast<uint64_t>(w) * width, pop_off[a + 1]);
@@ -361,8 +359,10 @@ int Engine::build_local_tables() {
     DTB_TRY(dalloc(woff, rb, false));
     DTB_TRY(dalloc(pop_loc, P, false));
     DTB_TRY(dalloc(win_tab, wins.size(), false));
-    DTB_TRY(dalloc(local_scratch, 2 * wins.size() + 3));
+    DTB_TRY(dalloc(pop_win, P, false));
+    DTB_TRY(dalloc(local_scratch, local_scratch_words(wins.size())));
     DTB_CU(cudaMemcpyAsync(pop_loc, loc.data(), sizeof(uint4) * P, cudaMemcpyHostToDevice, stream));
+    DTB_CU(cudaMemcpyAsync(pop_win, first.data(), sizeof(uint2) * P, cudaMemcpyHostToDevice, stream));
     DTB_CU(cudaMemcpyAsync(win_tab, wins.data(), sizeof(uint4) * wins.size(), cudaMemcpyHostToDevice, stream));
     DTB_CU(build_local_offsets(out_ptr, out_col, out_w, static_cast<int>(wtype), pop_off_dev, P, n, pop_loc, nullptr,
                                nullptr, own_seg, woff, nullptr, stream));
@@ -382,6 +382,7 @@ static int alloc_core(Engine& e) {
     DTB_TRY(e.dalloc(e.pop_dev, e.P));
     DTB_TRY(e.dalloc(e.pop_off_dev, e.P + 1));
     DTB_TRY(e.dalloc(e.out_deg, e.n_pad));
+    DTB_TRY(e.dalloc(e.pop_live, e.P));
     DTB_TRY(e.dalloc(e.bits0, e.n_words));
     DTB_TRY(e.dalloc(e.bits1, e.n_words));
     DTB_TRY(e.dalloc(e.clock, 1));
@@ -391,7 +392,7 @@ static int alloc_core(Engine& e) {
     DTB_TRY(e.dalloc(e.prefix_dev, 8));
     DTB_TRY(e.dalloc(e.list, e.n_pad, false));
     DTB_TRY(e.dalloc(e.list_count, 1));
-    DTB_TRY(e.dalloc(e.list_ticket, 1));
+    DTB_TRY(e.dalloc(e.list_published, 2));
     {
         // population of the first neuron of every 1024-neuron LIF tile
         const uint32_t tiles = e.n_pad / kLifTile;
@@ -958,7 +959,7 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
     if (record) kflags |= kFlagRecord;
     if (!pull) kflags |= kFlagList;
     if (injected) kflags |= kFlagInjected;
-    const LaunchBatch b = single_batch();
+    LaunchBatch b = single_batch();
     const int pm = static_cast<int>(rq.prop_mode);
     const int wt = static_cast<int>(wtype);
     const bool time_k = (rq.flags & DTB_RUN_TIME_KERNELS) != 0;
@@ -997,6 +998,10 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
             return DTB_OK;
         };
         // the chunk's launches; `tuning` false while a graph is being captured
+        // the LIF kernel prepares the windows' work units when this chunk's pushes (or the tuner's) read them
+        const bool tune_here = tune_at >= done && tune_at < done + rows;
+        b.local.flush_reds = acc == ACC_FIXED ? 2u : 1u;
+        b.local.windows = acc != ACC_EXACT && (push_cfg.kind == PUSH_LOCAL || tune_here) ? n_windows : 0u;
         auto issue = [&](bool tuning) -> int {
             for (uint32_t s = 0; s < rows; ++s) {
                 const bool first = (done + s) == 0;
@@ -1016,7 +1021,6 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
                     if (!push_tuned[acc]) tune_at = tune_acc[acc].next_step(tune_at);
                 }
                 DTB_TRY(timed_launch(1, [&] { return launch_push(b, acc, wt, push_cfg, push_ctas, stream); }));
-                chunk_launches += push_extra_launches(b, acc, push_cfg);
                 if (isyn_any) DTB_TRY(timed_launch(3, [&] { return launch_stat_isyn(b, acc, sm_count, stream); }));
             }
             if (last_chunk && (acc == ACC_EXACT || acc == ACC_FIXED) && !pull)
@@ -1028,15 +1032,16 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
         bool eager_graphable = false;
         // a push chunk with no tuning pending and no per-kernel timing: replay its graph once its
         // shape has been seen before (the kernels read every per-run value from device memory)
-        const bool graphable = use_graph && !pull && !time_k && !(tune_at >= done && tune_at < done + rows);
+        const bool graphable = use_graph && !pull && !time_k && !tune_here;
         const uint64_t key[10] = {rows, kflags, static_cast<uint64_t>(pm), rq.syn_mode,
-                                  static_cast<uint64_t>(push_cfg.kind) * 100000 + push_cfg.param * 100 + push_cfg.lpr,
+                                  static_cast<uint64_t>(push_cfg.kind) * 100000 + push_cfg.param * 100 + push_cfg.lpr +
+                                      (static_cast<uint64_t>(b.local.dense_min) << 32),
                                   push_ctas, done == 0, last_chunk, isyn_any, ts};
         if (graphable && graph && std::memcmp(key, graph_key, sizeof(key)) == 0) {
             DTB_CU(cudaGraphLaunch(graph, stream));
             ++graph_launches;
             // launches of the replayed chunk, counted as the eager path does
-            chunk_launches = rows * (ts + 1u + push_extra_launches(b, acc, push_cfg) + (isyn_any ? 1u : 0u)) +
+            chunk_launches = rows * (ts + 1u + (isyn_any ? 1u : 0u)) +
                              (last_chunk && acc != ACC_FLOAT ? 1u : 0u);
         } else if (graphable && std::memcmp(key, seen_key, sizeof(key)) == 0 && ++seen_count >= 2 &&
                    seen_ms_per_step < kGraphMaxMsPerStep) {
@@ -1107,15 +1112,19 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
 // 5M network local:8 and local:2008 come within 1-3 % of each other on the sampled
 // bursts, while over whole runs local:2008 is 6.6 % faster (push 0.548 vs 0.585 ms).
 constexpr float kTuneTie = 0.02f;
-static void pick_best(TuneResult& res) {
+static void pick_best(TuneResult& res, uint32_t dense_min) {
     if (res.report.empty()) { res.best_ms = 0.0f; return; }
+    // A network whose peak stays below the windows' threshold only ever scatters: the window
+    // kernel and its preparation would cost it 1 to 2 us a step for nothing.
+    auto barred = [&](const TuneEntry& t) { return t.cfg.kind == PUSH_LOCAL && res.peak < dense_min; };
     float fastest = 1e30f;
-    for (const TuneEntry& t : res.report) fastest = std::min(fastest, t.ms);
+    for (const TuneEntry& t : res.report)
+        if (!barred(t)) fastest = std::min(fastest, t.ms);
     const TuneEntry* pick = nullptr;
     for (const TuneEntry& t : res.report) {
-        if (t.ms > fastest * (1.0f + kTuneTie)) continue;
-        const bool preferred = t.cfg.kind == PUSH_LOCAL && t.cfg.param == kLocalConcurrent;
-        if (!pick || (preferred && !(pick->cfg.kind == PUSH_LOCAL && pick->cfg.param == kLocalConcurrent))) pick = &t;
+        if (barred(t) || t.ms > fastest * (1.0f + kTuneTie)) continue;
+        const bool preferred = t.cfg.kind == PUSH_LOCAL && t.cfg.param == kLocalConcurrent2;
+        if (!pick || (preferred && !(pick->cfg.kind == PUSH_LOCAL && pick->cfg.param == kLocalConcurrent2))) pick = &t;
     }
     res.best = pick->cfg;
     res.best_ms = pick->ms;
@@ -1127,7 +1136,7 @@ static void pick_best(TuneResult& res) {
 int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int acc, int wtype, int sm_count,
                     cudaStream_t stream, cudaEvent_t ev[2], TuneResult& res) {
     uint32_t count = 0;
-    DTB_CU(cudaMemcpyAsync(&count, b.spikes.count, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    DTB_CU(cudaMemcpyAsync(&count, b.spikes.published, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
     DTB_CU(cudaStreamSynchronize(stream));
     uint64_t total_n = 0;
     for (const NetView& v : views) total_n += v.n_pad;
@@ -1138,7 +1147,7 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         if (res.observed >= res.observe + kTuneGiveUp) {
             // settle: the best of the samples so far, or the default variant
             res.tuned = true;
-            pick_best(res);
+            pick_best(res, b.local.dense_min);
         }
         return DTB_OK;
     }
@@ -1151,6 +1160,16 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         cudaFree(scratch);
         return cuda_fail(cudaErrorMemoryAllocation, "tune_push");
     }
+    // Between replays L2 is overwritten: in a run a step's rows come from DRAM, while a replay of a
+    // step of some ten MB would find them in L2 and favour the variants with little in flight (on a
+    // 12-member batch the window form, measured warm, was kept although it ran 36 % slower).
+    // Without room for the buffer the replays run warm.
+    constexpr size_t kFlushBytes = 192ull << 20;
+    void* flush = nullptr;
+    if (cudaMalloc(&flush, kFlushBytes) != cudaSuccess) {
+        cudaGetLastError();
+        flush = nullptr;
+    }
     std::vector<NetView> tv(views);
     size_t off = 0;
     for (NetView& v : tv) {
@@ -1161,18 +1180,23 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         off += v.n_pad;
     }
     std::vector<TuneEntry> step;
+    // the window kernel's counters, used up by each launch
+    auto reset_units = [&]() -> cudaError_t {
+        return b.local.windows ? cudaMemsetAsync(b.local.scratch + 2 * b.local.windows + 1, 0, 2 * sizeof(uint32_t), stream) : cudaSuccess;
+    };
     auto body = [&]() -> int {
         DTB_CU(cudaMemcpyAsync(tview, tv.data(), sizeof(NetView) * tv.size(), cudaMemcpyHostToDevice, stream));
         DTB_CU(cudaMemsetAsync(scratch, 0, per * total_n, stream));
         LaunchBatch tb = b;
         tb.nets = tview;
         for (const PushCfg& c : kPushCands) {
-            if (c.kind == PUSH_LOCAL && (acc == ACC_EXACT || b.windows_total == 0)) continue;
+            if (c.kind == PUSH_LOCAL && (acc == ACC_EXACT || b.local.windows == 0)) continue;
             uint32_t ctas = 0;
             DTB_CU(push_prepare(acc, wtype, c, sm_count, &ctas));
             float ms_min = 1e30f;
             for (int rep = 0; rep < 3; ++rep) {
-                set_u32_kernel<<<1, 1, 0, stream>>>(b.spikes.count, count);
+                DTB_CU(reset_units());
+                if (flush) DTB_CU(cudaMemsetAsync(flush, rep, kFlushBytes, stream));
                 DTB_CU(cudaEventRecord(ev[0], stream));
                 DTB_CU(launch_push(tb, acc, wtype, c, ctas, stream));
                 DTB_CU(cudaEventRecord(ev[1], stream));
@@ -1183,14 +1207,14 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
             }
             step.push_back({c, ms_min});
         }
-        set_u32_kernel<<<1, 1, 0, stream>>>(b.spikes.count, count);
-        DTB_CU(cudaGetLastError());
+        DTB_CU(reset_units());
         return DTB_OK;
     };
     const int st = body();
     cudaStreamSynchronize(stream);
     cudaFree(scratch);
     cudaFree(tview);
+    if (flush) cudaFree(flush);
     if (st != DTB_OK) return st;
     // running mean per variant over the samples
     if (res.report.size() != step.size()) {
@@ -1203,7 +1227,7 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
     }
     if (res.samples < res.want) return DTB_OK;
     res.tuned = true;
-    pick_best(res);
+    pick_best(res, b.local.dense_min);
     return DTB_OK;
 }
 
@@ -1215,7 +1239,7 @@ int Engine::tune_push(const LaunchBatch& b, int acc) {
     TuneResult& res = tune_acc[acc];
     DTB_TRY(tune_push_views(b, {view}, acc, static_cast<int>(wtype), sm_count, stream, tune_ev, res));
     if (!res.tuned) return DTB_OK;
-    push_cfg = res.best;
+    if (!res.report.empty()) push_cfg = res.best;
     push_tuned[acc] = true;
     tuned_ms = res.best_ms;
     tune_report = res.report;
@@ -1685,6 +1709,7 @@ int32_t dtb_set_push_variant(void* engine, int32_t kind, int32_t param) {
     Engine* e = as_engine(engine);
     if (kind < 0) {
         e->autotune = true;
+        e->window_always = false;
         for (int a = 0; a < 3; ++a) {
             e->push_tuned[a] = false;
             e->tune_acc[a].reset();
@@ -1695,6 +1720,7 @@ int32_t dtb_set_push_variant(void* engine, int32_t kind, int32_t param) {
     if (!dtb::push_cfg_from_abi(kind, param, cfg)) return dtb::fail(DTB_INVALID_PARAMETER, "unknown push variant");
     e->push_cfg = cfg;
     e->autotune = false;
+    e->window_always = true;
     return DTB_OK;
 }
 

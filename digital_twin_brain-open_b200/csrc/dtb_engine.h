@@ -54,7 +54,6 @@ struct TuneResult {
 };
 bool push_cfg_from_abi(int kind, int param, PushCfg& cfg);
 __global__ void set_u64_kernel(unsigned long long* p, unsigned long long v);
-__global__ void set_u32_kernel(uint32_t* p, uint32_t v);
 // Reads the live spike count and, when the step qualifies as a sample (TuneResult),
 // times every push variant on it and adds the times to `res`.  A list of fewer than
 // 0.2 % of the neurons never qualifies.
@@ -113,8 +112,6 @@ public:
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaStream_t aux = nullptr;                            // second stream of the concurrent local push
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     float dt = 0.1f;
     uint32_t wtype = W_F32;
     uint64_t seed = 0;
@@ -190,7 +187,7 @@ public:
     uint32_t* prefix_dev = nullptr;   // [lif 2][pull 2][vbase 2][local windows 2]
     uint32_t* list = nullptr;
     uint32_t* list_count = nullptr;
-    uint32_t* list_ticket = nullptr;
+    uint32_t* list_published = nullptr;
     uint32_t* tile_pop = nullptr;
     uint32_t lif_ctas_per_sm = kLifCtasPerSm;
     // population-local push tables (built when every out-degree row is sorted)
@@ -198,14 +195,17 @@ public:
     uint32_t* woff = nullptr;
     uint4* pop_loc = nullptr;
     uint4* win_tab = nullptr;
+    uint2* pop_win = nullptr;
+    uint32_t* pop_live = nullptr;
     uint32_t n_windows = 0;
-    uint32_t* local_scratch = nullptr;   // [2 * n_windows + 3] per-step unit bookkeeping (zeroed)
+    uint32_t* local_scratch = nullptr;   // [local_scratch_words(n_windows)] per-step unit bookkeeping (zeroed)
     int build_local_tables();
 
     // push kernel variant (autotuned on the first active run)
     PushCfg push_cfg{PUSH_REG, 8, 32};
     uint32_t push_ctas = 0;
     bool autotune = true;
+    bool window_always = false;           // a window form chosen by the caller takes the windows in every step
     bool push_tuned[3] = {false, false, false};
     TuneResult tune_acc[3];               // samples gathered so far (float, exact and fixed push)
     float tuned_ms = 0.0f;

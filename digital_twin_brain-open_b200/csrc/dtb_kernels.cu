@@ -309,15 +309,16 @@ __device__ __forceinline__ void lif_prefetch(const NetView* __restrict__ nets, c
 }
 
 // thread 0: the CTA finished `cnt` tiles of `nv`; the last CTA of the network advances its clock
-__device__ __forceinline__ void lif_ticket(const NetView& nv, uint32_t cnt, float t, unsigned long long n) {
+// (returns 1 then, else 0)
+__device__ __forceinline__ uint32_t lif_ticket(const NetView& nv, uint32_t cnt, float t, unsigned long long n) {
     __threadfence();
     const uint32_t k = atomicAdd(nv.ticket, cnt);
-    if (k + cnt == nv.lif_tiles) {
-        nv.clock->t = t;
-        nv.clock->n = n;
-        *nv.ticket = 0u;
-        __threadfence();
-    }
+    if (k + cnt != nv.lif_tiles) return 0u;
+    nv.clock->t = t;
+    nv.clock->n = n;
+    *nv.ticket = 0u;
+    __threadfence();
+    return 1u;
 }
 
 // A CTA steps chunks of `chunk` consecutive tiles, chunks strided by the grid:
@@ -329,11 +330,14 @@ __device__ __forceinline__ uint32_t lif_next_tile(uint32_t gt, uint32_t chunk, u
     return (gt / chunk + gridDim.x) * chunk;
 }
 
+__device__ __forceinline__ void local_prep(const NetView* __restrict__ nets, const LocalPlan& lp, uint32_t n_nets, uint32_t count,
+                                           uint32_t* s_warp);
+
 template <int JM>
 __global__ void __launch_bounds__(kLifThreads, kLifCtasPerSm)
 lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_prefix,
            const uint32_t* __restrict__ vbase, uint32_t n_nets, uint32_t total_tiles, SpikeList sl, uint32_t flags,
-           int prop_mode, const uint32_t* __restrict__ tile_net, uint32_t chunk) {
+           int prop_mode, const uint32_t* __restrict__ tile_net, uint32_t chunk, LocalPlan lp) {
     extern __shared__ __align__(128) float lsm[];
     __shared__ __align__(8) uint64_t s_bar[kLifStages];
     // population slots of the statistics, by tile parity: tile `it` adds into set it & 1,
@@ -362,6 +366,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     __shared__ float s_tk_t[kTicketSlots];
     __shared__ unsigned long long s_tk_n[kTicketSlots];
     uint32_t n_tk = 0;                 // thread 0's count of table entries
+    uint32_t nets_done = 0;            // networks this CTA was the last to finish (thread 0)
     if (tid < 2 * kStatSlots) { s_cnt[tid / kStatSlots][tid % kStatSlots] = 0; s_vs[tid / kStatSlots][tid % kStatSlots] = 0; }
     if (tid == 0) {
         for (int s = 0; s < kLifStages; ++s) mbar_init(&s_bar[s], 1);
@@ -386,7 +391,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
             // read-only cache, so switching needs no barrier)
             if (tid == 0 && done_here) {
                 if (n_tk == kTicketSlots) {
-                    for (uint32_t q = 0; q < n_tk; ++q) lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
+                    for (uint32_t q = 0; q < n_tk; ++q) nets_done += lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
                     n_tk = 0;
                 }
                 s_tk_net[n_tk] = cur_net;
@@ -545,10 +550,11 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         // ---- spike bitmaps and list: step k of a warp covers one 32-neuron word
         //      (propagated: parity buffer and one slot range per warp in the list;
         //      threshold: history row)
+        uint32_t wtotal = 0;               // neurons of the warp new to the step's list
         {
             uint32_t* bits = parity ? nv.bits1 : nv.bits0;
             const uint32_t word0 = (tile_first >> 5) + (tid >> 5);
-            uint32_t wprop[4], wtotal = 0;
+            uint32_t wprop[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint32_t all = __ballot_sync(0xffffffffu, (nib_prop >> k) & 1u);
@@ -575,6 +581,22 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
                     if ((nib_prop >> k) & 1u) sl.list[base + __popc(wprop[k] & below)] = vb + kSlotsPerTile * k;
                     base += __popc(wprop[k]);
                 }
+                // spiking rows per population, for the windows: one reduction per warp, or per
+                // neuron in the few warps that hold a population boundary
+                if (lp.windows) {
+                    const uint32_t pa = __shfl_sync(0xffffffffu, p_first, 0), pb = __shfl_sync(0xffffffffu, p, 31);
+                    if (pa == pb) {
+                        if (lane == 0) atomicAdd(nv.pop_live + pa, wtotal);
+                    } else {
+                        uint32_t pk = p_first;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (!((wprop[k] >> lane) & 1u)) continue;
+                            while (pk + 1 < nv.n_pops && __ldg(nv.pop_off + pk + 1) <= i0 + kSlotsPerTile * k) ++pk;
+                            atomicAdd(nv.pop_live + pk, 1u);
+                        }
+                    }
+                }
             }
         }
         // ---- population statistics: one sum per warp when the warp's neurons share a
@@ -591,7 +613,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
                 warp_stat_segments(nv, sa, row, p_first + 1, cnt_nxt != 0 || vs_nxt != 0, cnt_nxt, vs_nxt, lane);
             }
         }
-        const unsigned long long wev = warp_sum_ull(ev);
+        const unsigned long long wev = wtotal ? warp_sum_ull(ev) : 0ull;
         if (lane == 0 && wev) atomicAdd(nv.events, wev);
 
         // barrier B: the stage holds the finished tile; store it, flush statistics
@@ -626,8 +648,28 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     // the CTA's last stores complete before its tiles count towards the clock
     if (tid == 0) {
         bulk_wait_all();
-        for (uint32_t q = 0; q < n_tk; ++q) lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
-        if (done_here) lif_ticket(nets[cur_net], done_here, t_last_tile, n_last_tile);
+        for (uint32_t q = 0; q < n_tk; ++q) nets_done += lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
+        if (done_here) nets_done += lif_ticket(nets[cur_net], done_here, t_last_tile, n_last_tile);
+    }
+    // the CTA that finishes the launch's last network hands the step's list to the push kernel,
+    // empties it for the next step, and prepares the windows' work units
+    if ((flags & kFlagList) && last_sub) {
+        __shared__ uint32_t s_warp[33];
+        __shared__ uint32_t s_published;               // list length + 1 in the last CTA, else 0
+        if (tid == 0) {
+            s_published = 0u;
+            if (nets_done && (n_nets == 1 || atomicAdd(sl.published + 1, nets_done) + nets_done == n_nets)) {
+                const uint32_t c = __ldcg(sl.count);
+                sl.published[0] = c;
+                sl.published[1] = 0u;
+                *sl.count = 0u;
+                s_published = c + 1u;
+            }
+        }
+        if (lp.windows) {
+            __syncthreads();
+            if (s_published) local_prep(nets, lp, n_nets, s_published - 1u, s_warp);
+        }
     }
 }
 
@@ -652,131 +694,121 @@ __device__ __forceinline__ void prefetch_span_l2(const uint32_t* col, const void
 // ---------------------------------------------------------------------------
 // Push propagation: one warp per spiking row of the out-degree CSR
 // ---------------------------------------------------------------------------
-template <int ACC, int WT, int kPushUnroll, int LPR, int LOCAL>
+// Where a network's spikes land.
+struct PushDst {
+    float4* J;
+    long long* dJ;
+    unsigned long long* dJf;
+    float fscale;
+};
+template <int ACC>
+__device__ __forceinline__ PushDst push_dst(const NetView& nv) { return PushDst{nv.J, nv.dJ, nv.dJf, nv.fix_scale}; }
+
+template <int ACC>
+__device__ __forceinline__ void reduce_synapse(const PushDst& d, uint32_t c, float2 w, unsigned long long keep) {
+    const uint32_t target = c & kIndexMask, kind = c >> 31;
+    if constexpr (ACC == ACC_FLOAT) {
+        red_add_f32x2_keep(reinterpret_cast<float2*>(d.J + target) + kind, w, keep);
+    } else if constexpr (ACC == ACC_FIXED) {
+        red_add_u64_keep(d.dJf + 2ull * target + kind, pack_fixed(w, d.fscale), keep);
+    } else {
+        unsigned long long* q = reinterpret_cast<unsigned long long*>(d.dJ) + static_cast<size_t>(target) * 4 + 2 * kind;
+        red_add_u64(q, static_cast<unsigned long long>(float_to_fix(w.x)));
+        red_add_u64(q + 1, static_cast<unsigned long long>(float_to_fix(w.y)));
+    }
+}
+
+// Synapses at virtual positions x0, x0 + step, ... of [0, len): position x is CSR slot
+// beg + x below len1 and beg2 + (x - len1) from there on (LOCAL: the own-population span
+// between the two is left out); U positions LPR apart are in flight per lane.
+template <int ACC, int WT, int U, int LPR, bool LOCAL>
+__device__ __forceinline__ void push_span(const uint32_t* col, const void* wts, const PushDst& d, unsigned long long beg,
+                                          uint32_t len1, unsigned long long beg2, uint32_t len, uint32_t x0, uint32_t step,
+                                          unsigned long long keep) {
+    for (uint32_t x = x0; x < len; x += step) {
+        uint32_t c[U];
+        float2 w[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const uint32_t xq = x + static_cast<uint32_t>(LPR) * q;
+            if (xq < len) {
+                const unsigned long long idx = LOCAL ? (xq < len1 ? beg + xq : beg2 + (xq - len1)) : beg + xq;
+                c[q] = __ldcs(col + idx);
+                w[q] = load_weight<WT>(wts, idx);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (x + static_cast<uint32_t>(LPR) * q < len) reduce_synapse<ACC>(d, c[q], w[q], keep);
+    }
+}
+
+// Whole rows of the spike list, LPR lanes per row: 32 (a warp per row) or 16 / 8 (2 / 4 rows
+// per warp, for short rows).  With fewer rows than groups of lanes, a row is cut into
+// interleaved parts of U x LPR synapses so that a quiet step (a few dozen rows, most of the
+// steps of a bursting network) is one round of loads deep instead of one per U x LPR synapses.
+template <int ACC, int WT, int U, int LPR>
 __device__ __forceinline__ void push_rows(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets,
-                                          SpikeList sl) {
-    // LPR lanes per row: 32 (a warp per row) or 16 / 8 (2 / 4 rows per warp, for short rows).
-    // LOCAL: the own-population span of a row (own_seg) is left to push_local_kernel.
+                                          const SpikeList& sl, uint32_t count) {
     constexpr uint32_t kGroups = 32 / LPR;
-    const uint32_t count = *sl.count;
+    constexpr uint32_t kMaxParts = 8;
     const uint32_t lane = (threadIdx.x & 31u) % LPR;
     const uint32_t gw = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kGroups + (threadIdx.x & 31u) / LPR;
     const uint32_t nw = ((gridDim.x * blockDim.x) >> 5) * kGroups;
-    const unsigned long long* ptr = nets[0].out_ptr;
+    const uint32_t parts = count ? min(kMaxParts, max(1u, nw / count)) : 1u;
+    const uint32_t total = count * parts;            // below nw, or count itself
     const uint32_t* col = nets[0].out_col;
     const void* wts = nets[0].out_w;
-    float4* J = nets[0].J;
-    long long* dJ = nets[0].dJ;
-    unsigned long long* dJf = nets[0].dJf;
-    float fscale = nets[0].fix_scale;
-    const uint2* own = LOCAL ? nets[0].own_seg : nullptr;
+    const unsigned long long* ptr = nets[0].out_ptr;
+    PushDst d = push_dst<ACC>(nets[0]);
     const unsigned long long keep = l2_policy_keep();
     uint32_t vb = 0;
-    for (uint32_t r = gw; r < count; r += nw) {
-        const uint32_t v = __ldg(sl.list + r);
+    for (uint32_t r = gw; r < total; r += nw) {
+        const uint32_t row = parts > 1 ? r / parts : r, part = r - row * parts;
+        const uint32_t v = __ldg(sl.list + row);
         if (n_nets > 1) {
             const uint32_t k = find_net(vbase, n_nets, v);
             vb = __ldg(vbase + k);
             ptr = nets[k].out_ptr;
             col = nets[k].out_col;
             wts = nets[k].out_w;
-            J = nets[k].J;
-            dJ = nets[k].dJ;
-            dJf = nets[k].dJf;
-            fscale = nets[k].fix_scale;
-            if constexpr (LOCAL) own = nets[k].own_seg;
+            d = push_dst<ACC>(nets[k]);
         }
         const uint32_t j = v - vb;
-        const unsigned long long beg = __ldg(ptr + j), end = __ldg(ptr + j + 1);
-        // virtual positions [0, len): [0, len1) -> beg + x, [len1, len) -> beg2 + (x - len1)
-        unsigned long long len1 = end - beg, beg2 = end;
-        if constexpr (LOCAL) {
-            if (own) {
-                const uint2 o = __ldg(own + j);
-                len1 = o.x;
-                beg2 = beg + o.y;
-            }
-        }
-        const unsigned long long len = len1 + (end - beg2);
-        for (unsigned long long x = lane; x < len; x += static_cast<unsigned long long>(LPR) * kPushUnroll) {
-            uint32_t c[kPushUnroll];
-            float2 w[kPushUnroll];
-#pragma unroll
-            for (int q = 0; q < kPushUnroll; ++q) {
-                const unsigned long long xq = x + static_cast<unsigned long long>(LPR) * q;
-                if (xq < len) {
-                    const unsigned long long idx = LOCAL ? (xq < len1 ? beg + xq : beg2 + (xq - len1)) : beg + xq;
-                    c[q] = __ldcs(col + idx);
-                    w[q] = load_weight<WT>(wts, idx);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < kPushUnroll; ++q) {
-                const unsigned long long xq = x + static_cast<unsigned long long>(LPR) * q;
-                if (xq < len) {
-                    const uint32_t target = c[q] & kIndexMask;
-                    const uint32_t kind = c[q] >> 31;
-                    if constexpr (ACC == ACC_FLOAT) {
-                        red_add_f32x2_keep(reinterpret_cast<float2*>(J + target) + kind, w[q], keep);
-                    } else if constexpr (ACC == ACC_FIXED) {
-                        red_add_u64_keep(dJf + 2ull * target + kind, pack_fixed(w[q], fscale), keep);
-                    } else {
-                        unsigned long long* d = reinterpret_cast<unsigned long long*>(dJ) + static_cast<size_t>(target) * 4 + 2 * kind;
-                        red_add_u64(d, static_cast<unsigned long long>(float_to_fix(w[q].x)));
-                        red_add_u64(d + 1, static_cast<unsigned long long>(float_to_fix(w[q].y)));
-                    }
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(sl.ticket, 1u) == gridDim.x - 1) {
-            *sl.count = 0u;
-            *sl.ticket = 0u;
-            __threadfence();
-        }
+        const unsigned long long beg = __ldg(ptr + j);
+        const uint32_t len = static_cast<uint32_t>(__ldg(ptr + j + 1) - beg);
+        push_span<ACC, WT, U, LPR, false>(col, wts, d, beg, len, 0ull, len, lane + part * (LPR * U), parts * (LPR * U), keep);
     }
 }
 
-template <int ACC, int WT, int kPushUnroll, int LPR, int LOCAL = 0>
+template <int ACC, int WT, int U, int LPR>
 __global__ void __launch_bounds__(kPushThreads)
 push_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets, SpikeList sl) {
-    push_rows<ACC, WT, kPushUnroll, LPR, LOCAL>(nets, vbase, n_nets, sl);
-}
-
-// The cross-population part held to 64 registers (4 CTAs of 256 threads) for local:2016: two
-// CTAs of it and the 512-thread window kernel (64 registers) fill exactly the SM's 65,536
-// registers, so the two kernels really share every SM; at the 80 registers the compiler picks
-// otherwise, a window CTA cannot start on an SM until the cross-population CTAs there have
-// finished.  local:2008 keeps that 80-register form: held to 64 it also shared its SMs but ran
-// 2 % slower on burst steps and no faster over whole runs of the regional network.
-template <int ACC, int WT>
-__global__ void __launch_bounds__(kPushThreads, 4)
-push_kernel_cross64(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets, SpikeList sl) {
-    push_rows<ACC, WT, 8, 32, 1>(nets, vbase, n_nets, sl);
+    push_rows<ACC, WT, U, LPR>(nets, vbase, n_nets, sl, *sl.published);
 }
 
 // ---------------------------------------------------------------------------
-// Population-local push, phase B.  Each population with local windows is cut
-// into windows of at most kLocalWin neurons; a row's synapses into one window
-// are a contiguous span (rows are sorted by postsynaptic neuron) between two
-// woff boundaries.  The work of a step is split into units of up to
-// kLocalUnitRows spiking rows of one window's population:
+// Population-window push.  Each population with local windows is cut into windows
+// of at most kLocalWin neurons; a row's synapses into one window are a contiguous
+// span (rows are sorted by postsynaptic neuron) between two woff boundaries.
 //
-//   local_prep_kernel    spiking rows of each window's population (bitmap popcount);
-//                        its last block turns them into the units' exclusive prefix
-//                        and resets the unit counter
-//   push_local_kernel    persistent, one 1024-thread CTA per SM: takes units from an
-//                        atomic counter, finds the unit's rows by a block-wide prefix
-//                        over the population's bitmap, sums their window spans into
-//                        shared memory, and flushes the window to J with coalesced
-//                        red.global.add.v4.f32 when it moves to another window.
+// One persistent kernel, one 1024-thread CTA per SM, takes a step in one of two ways:
+//
+// * a step of few events (the LIF kernel's last CTA left no units): every warp walks
+//   whole rows of the spike list with scattered L2 reductions, as push_kernel does;
+// * a busy step: the first win_warps warps of each CTA take work units -- up to
+//   kLocalUnitRows spiking rows of one window's population -- from an atomic counter,
+//   sum their spans into the window's sums in shared memory and flush them to J with
+//   coalesced red.global.add.v4.f32 when they move to another window, while the other
+//   warps take chunks of the spike list from a second counter and scatter the rows'
+//   cross-population synapses with L2 reductions.  Warps that run out of units help
+//   with the chunks, so both ends of the step finish together.
 //
 // A bursting population becomes many units spread over every SM, so the step is
 // balanced whatever the activity pattern; the L2 sees one 16-byte reduction per
-// touched neuron per flush instead of one per synapse.
+// touched neuron per flush instead of one per synapse.  Bursting networks spend most of
+// their steps quiet: on the 200k-neuron regional network 196 of 200 steps deliver tens of
+// rows, and a window pass in each of them cost about 30 us against 5 us for the rows.
 //
 // The window sums are 32-bit fixed point: w is rounded to a multiple of 2^-s and
 // added with red.shared.add.u32 (native, fire-and-forget; a shared-memory float
@@ -786,38 +818,43 @@ push_kernel_cross64(const NetView* __restrict__ nets, const uint32_t* __restrict
 // spikes.  The regional network gets s = 21 (resolution 4.8e-7, below the
 // rounding of float atomics onto J of order 10).
 // ---------------------------------------------------------------------------
-constexpr int kLocalThreads = 1024;
-constexpr int kLocalThreadsShared = 768;   // window kernel beside a cross-population CTA on the same SM
-constexpr int kLocalThreadsShared2 = 512;  // ... beside two
+constexpr int kWindowThreads = 1024;        // one CTA per SM, 64 registers a thread
 constexpr int kLocalUnroll = 8;
 constexpr uint32_t kLocalUnitRows = 1024;   // spiking rows per work unit (measured: 256 / 512 / 1024 rows -> push 0.596 / 0.561 / 0.548 ms at 5M)
+constexpr uint32_t kLocalUnitLeast = 64;
+constexpr uint32_t kCrossChunk = 8;         // most list rows a warp takes at a time for their cross-population synapses
 constexpr size_t kLocalSmem = 4ull * kLocalWin * sizeof(int) + kLocalUnitRows * (2 * sizeof(uint32_t) + sizeof(unsigned long long));
 
 __device__ __forceinline__ void red_add_shared_u32(const void* p, uint32_t v) {
     asm volatile("red.shared.add.u32 [%0], %1;" :: "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(v) : "memory");
 }
 
+// Barrier 1 among the first nt threads of the CTA (nt a multiple of 32).
+__device__ __forceinline__ void group_sync(uint32_t nt) { asm volatile("bar.sync 1, %0;" :: "r"(nt) : "memory"); }
+
 // Spiking-row bitmap word wi of the population [p_lo, p_hi), bits outside masked off.
-__device__ __forceinline__ uint32_t pop_word(const uint32_t* bits, uint32_t wi, uint32_t p_lo, uint32_t p_hi) {
-    uint32_t m = bits[wi];
+__device__ __forceinline__ uint32_t pop_mask(uint32_t m, uint32_t wi, uint32_t p_lo, uint32_t p_hi) {
     const uint32_t b0 = wi << 5;
     if (b0 < p_lo) m &= ~0u << (p_lo - b0);
     if (p_hi - b0 < 32u) m &= (1u << (p_hi - b0)) - 1u;
     return m;
 }
+__device__ __forceinline__ uint32_t pop_word(const uint32_t* bits, uint32_t wi, uint32_t p_lo, uint32_t p_hi) {
+    return pop_mask(bits[wi], wi, p_lo, p_hi);
+}
 
-// Exclusive prefix of v over the block (blockDim.x a multiple of 32); *total = sum.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Exclusive prefix of v over the CTA's first nt threads; *total = sum.
+__device__ __forceinline__ uint32_t group_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t* total, uint32_t nt) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = nt >> 5;
     uint32_t incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= static_cast<uint32_t>(o)) incl += y;
     }
-    __syncthreads();
+    group_sync(nt);
     if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
+    group_sync(nt);
     if (warp == 0) {
         uint32_t x = lane < nw ? s_warp[lane] : 0u;
         uint32_t xi = x;
@@ -829,14 +866,14 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
         if (lane < nw) s_warp[lane] = xi - x;
         if (lane == 31) s_warp[32] = xi;
     }
-    __syncthreads();
+    group_sync(nt);
     *total = s_warp[32];
     return s_warp[warp] + incl - v;
 }
 
 struct LocalWindow {
     const NetView* nv;
-    uint32_t a, lo, hi, k, ka1, p_lo, p_hi;
+    uint32_t a, lo, hi, k, ka1, p_lo, p_hi, least;
     unsigned long long rb_k;
     float scale, unscale;
 };
@@ -858,49 +895,72 @@ __device__ __forceinline__ void load_window(const NetView* __restrict__ nets, co
     W.rb_k = (static_cast<unsigned long long>(pl.z) | (static_cast<unsigned long long>(pl.w) << 32)) + W.k;
     W.p_lo = __ldg(W.nv->pop_off + W.a);
     W.p_hi = __ldg(W.nv->pop_off + W.a + 1);
+    W.least = __ldg(W.nv->pop_win + W.a).y;
 }
 
-// scratch: [windows] spiking rows of each window's population, [windows + 1]
-// unit prefix, [1] unit counter, [1] block ticket.  One block per window counts
-// its population's spiking rows; the last block to finish (ticket) turns the
-// counts into the unit prefix and resets the counter, so the window kernel that
-// follows needs one launch before it instead of a count and a scan.
-__global__ void __launch_bounds__(256)
-local_prep_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ win_prefix, uint32_t n_nets,
-                  uint32_t windows, uint32_t* scratch) {
-    __shared__ uint32_t s_warp[33];
-    __shared__ uint32_t s_last;
-    LocalWindow W;
-    load_window(nets, win_prefix, n_nets, blockIdx.x, W);
-    const uint32_t* bits = (W.nv->clock->n & 1ull) ? W.nv->bits1 : W.nv->bits0;
-    uint32_t c = 0;
-    for (uint32_t wi = (W.p_lo >> 5) + threadIdx.x; wi < ((W.p_hi + 31) >> 5); wi += blockDim.x)
-        c += __popc(pop_word(bits, wi, W.p_lo, W.p_hi));
-    uint32_t total;
-    block_exclusive_scan(c, s_warp, &total);
-    uint32_t* ticket = scratch + 2 * windows + 2;
+// Rows per work unit of a window: the step's unit size, not below the rows that pay for a
+// flush (`reds` reductions a neuron: 1 of 16 bytes onto J, 2 of 8 bytes onto dJf).
+__device__ __forceinline__ uint32_t unit_rows_of(uint32_t unit, uint32_t least, uint32_t reds) {
+    return min(kLocalUnitRows, max(unit, reds * least));
+}
+
+// Work units of a busy step, by the last CTA of the step's LIF launch.
+// scratch: [windows] spiking rows of each window's population, [windows + 1] unit prefix,
+// then the unit counter and the cross-population chunk counter, both zeroed here, and the rows
+// per unit: at most kLocalUnitRows, fewer when that gives the SMs too few units to even out.
+// A step below dense_min spikes gets a total of 0 units, which is all the push kernel reads.
+// In a busy step a population's windows are taken when its spiking rows pay for the flushes
+// (pop_win); the rows of the others (rows[] = 0) are scattered whole.
+// The LIF warps count their spikes per population as they list them (pop_live, emptied here
+// for the next step): counting the bitmap here took one CTA 30 us at 3M neurons, and in a
+// launch of its own it cost every step 5 to 8 us.
+__device__ __forceinline__ void local_prep(const NetView* __restrict__ nets, const LocalPlan& lp, uint32_t n_nets, uint32_t count,
+                                           uint32_t* s_warp) {
+    const uint32_t windows = lp.windows, nt = blockDim.x;
+    uint32_t* rows = lp.scratch;
+    uint32_t* upre = rows + windows;
     if (threadIdx.x == 0) {
-        scratch[blockIdx.x] = total;
-        __threadfence();
-        s_last = atomicAdd(ticket, 1u) == windows - 1;
+        upre[windows] = 0u;
+        upre[windows + 1] = 0u;
+        upre[windows + 2] = 0u;
+    }
+    const bool busy = count >= lp.dense_min;
+    uint32_t all = 0;
+    for (uint32_t i = threadIdx.x; busy && i < windows; i += nt) {
+        const uint32_t net = n_nets > 1 ? find_net(lp.win_prefix, n_nets, i) : 0u;
+        const NetView& nv = nets[net];
+        const uint32_t a = nv.win_tab[i - __ldg(lp.win_prefix + net)].x;
+        const uint32_t c = __ldcg(nv.pop_live + a);
+        const uint32_t r = lp.always || c >= __ldg(nv.pop_win + a).y ? c : 0u;
+        rows[i] = r;
+        all += r;
     }
     __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    uint32_t* upre = scratch + windows;
+    for (uint32_t k = 0; k < n_nets; ++k)
+        for (uint32_t p = threadIdx.x; p < nets[k].n_pops; p += nt) nets[k].pop_live[p] = 0u;
+    if (!busy) return;
+    // the unit size that spreads the step's rows over the SMs, then the windows' unit prefix
+    uint32_t sum;
+    group_exclusive_scan(all, s_warp, &sum, nt);
+    const uint32_t unit = min(kLocalUnitRows, max(kLocalUnitLeast, sum / lp.unit_target + 1u));
     uint32_t carry = 0;
-    for (uint32_t base = 0; base < windows; base += blockDim.x) {
+    for (uint32_t base = 0; base < windows; base += nt) {
         const uint32_t i = base + threadIdx.x;
-        const uint32_t u = i < windows ? (__ldcg(scratch + i) + kLocalUnitRows - 1) / kLocalUnitRows : 0u;
+        uint32_t u = 0;
+        if (i < windows) {
+            const uint32_t net = n_nets > 1 ? find_net(lp.win_prefix, n_nets, i) : 0u;
+            const NetView& nv = nets[net];
+            const uint32_t per = unit_rows_of(unit, __ldg(nv.pop_win + nv.win_tab[i - __ldg(lp.win_prefix + net)].x).y, lp.flush_reds);
+            u = (rows[i] + per - 1u) / per;
+        }
         uint32_t tot;
-        const uint32_t ex = block_exclusive_scan(u, s_warp, &tot);
+        const uint32_t ex = group_exclusive_scan(u, s_warp, &tot, nt);
         if (i < windows) upre[i] = carry + ex;
         carry += tot;
     }
     if (threadIdx.x == 0) {
         upre[windows] = carry;
-        upre[windows + 1] = 0u;      // the unit counter
-        *ticket = 0u;
+        upre[windows + 3] = unit;
     }
 }
 
@@ -909,13 +969,13 @@ local_prep_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__
 // fixed-mode units and go to dJf as two packed 64-bit integer reductions, so the
 // result does not depend on which CTA flushes first.
 template <bool FIX>
-__device__ __forceinline__ void local_flush(const LocalWindow& W, int* acc) {
-    __syncthreads();
+__device__ __forceinline__ void local_flush(const LocalWindow& W, int* acc, uint32_t nt) {
+    group_sync(nt);
     float4* J = W.nv->J + W.lo;
     unsigned long long* dJf = FIX ? W.nv->dJf + 2ull * W.lo : nullptr;
     const uint32_t width = W.hi - W.lo;
     const unsigned long long keep = l2_policy_keep();
-    for (uint32_t i = threadIdx.x; i < width; i += blockDim.x) {
+    for (uint32_t i = threadIdx.x; i < width; i += nt) {
         const int4 v = make_int4(acc[i], acc[kLocalWin + i], acc[2 * kLocalWin + i], acc[3 * kLocalWin + i]);
         if (v.x | v.y | v.z | v.w) {
             if constexpr (FIX) {
@@ -934,34 +994,34 @@ __device__ __forceinline__ void local_flush(const LocalWindow& W, int* acc) {
             acc[3 * kLocalWin + i] = 0;
         }
     }
-    __syncthreads();
+    group_sync(nt);
 }
 
-// launch bound of the full CTA for every NT: 64 registers, so the 768-thread form leaves a
-// 256-thread push CTA room on the SM
-template <int WT, int NT, int RL = 32, bool FIX = false>
-__global__ void __launch_bounds__(kLocalThreads, 1)
-push_local_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ win_prefix, uint32_t n_nets,
-                  uint32_t windows, uint32_t* scratch) {
+// The units' part of a busy step, by the CTA's first nt threads.  RL lanes per row: 32 (a
+// warp per row) or 16 (two rows per warp, for short spans).
+template <int WT, int RL, bool FIX>
+__device__ __forceinline__ void push_windows(const NetView* __restrict__ nets, const LocalPlan& lp, uint32_t n_nets,
+                                             uint32_t total_units, int* acc, uint32_t* s_warp, uint32_t* s_unit, uint32_t nt) {
     // plane c of kLocalWin 32-bit sums: random targets spread over all 32 banks
-    extern __shared__ int acc[];
     uint32_t* s_rows = reinterpret_cast<uint32_t*>(acc + 4 * kLocalWin);
     uint32_t* s_len = s_rows + kLocalUnitRows;
     unsigned long long* s_start = reinterpret_cast<unsigned long long*>(s_len + kLocalUnitRows);
-    __shared__ uint32_t s_warp[33];
-    __shared__ uint32_t s_unit;
-    const uint32_t* rows_of = scratch;
-    const uint32_t* upre = scratch + windows;
-    uint32_t* counter = scratch + 2 * windows + 1;
-    const uint32_t total_units = upre[windows];
+    const uint32_t windows = lp.windows;
+    const uint32_t* rows_of = lp.scratch;
+    const uint32_t* upre = rows_of + windows;
+    uint32_t* counter = lp.scratch + 2 * windows + 1;
+    const uint32_t unit = lp.scratch[2 * windows + 3];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint32_t i = threadIdx.x; i < 4 * kLocalWin; i += NT) acc[i] = 0;
+    {
+        int4* a4 = reinterpret_cast<int4*>(acc);
+        for (uint32_t i = threadIdx.x; i < kLocalWin; i += nt) a4[i] = make_int4(0, 0, 0, 0);
+    }
     LocalWindow W{};
     uint32_t cur = 0xFFFFFFFFu;
     for (;;) {
-        if (threadIdx.x == 0) s_unit = atomicAdd(counter, 1u);
-        __syncthreads();
-        const uint32_t u = s_unit;
+        if (threadIdx.x == 0) *s_unit = atomicAdd(counter, 1u);
+        group_sync(nt);
+        const uint32_t u = *s_unit;
         if (u >= total_units) break;
         // the unit's window: the last w with upre[w] <= u (windows without units repeat a value)
         uint32_t lo_w = 0, hi_w = windows - 1;
@@ -971,22 +1031,23 @@ push_local_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__
         }
         const uint32_t gw = lo_w;
         if (gw != cur) {
-            if (cur != 0xFFFFFFFFu) local_flush<FIX>(W, acc);
-            load_window(nets, win_prefix, n_nets, gw, W);
+            if (cur != 0xFFFFFFFFu) local_flush<FIX>(W, acc, nt);
+            load_window(nets, lp.win_prefix, n_nets, gw, W);
             if constexpr (FIX) W.scale = W.nv->fix_scale;   // sums in the network's fixed-mode units
             cur = gw;
         }
-        const uint32_t r_lo = (u - upre[gw]) * kLocalUnitRows;
-        const uint32_t r_hi = min(r_lo + kLocalUnitRows, rows_of[gw]);
-        // rows with population rank in [r_lo, r_hi): block prefix over the bitmap
+        const uint32_t unit_rows = unit_rows_of(unit, W.least, FIX ? 2u : 1u);
+        const uint32_t r_lo = (u - upre[gw]) * unit_rows;
+        const uint32_t r_hi = min(r_lo + unit_rows, rows_of[gw]);
+        // rows with population rank in [r_lo, r_hi): prefix over the population's bitmap
         const uint32_t* bits = (W.nv->clock->n & 1ull) ? W.nv->bits1 : W.nv->bits0;
         const uint32_t w_lo = W.p_lo >> 5, w_hi = (W.p_hi + 31) >> 5;
-        const uint32_t per = (w_hi - w_lo + NT - 1) / NT;
+        const uint32_t per = (w_hi - w_lo + nt - 1) / nt;
         const uint32_t my_lo = min(w_lo + threadIdx.x * per, w_hi), my_hi = min(my_lo + per, w_hi);
         uint32_t c = 0;
         for (uint32_t wi = my_lo; wi < my_hi; ++wi) c += __popc(pop_word(bits, wi, W.p_lo, W.p_hi));
         uint32_t total;
-        uint32_t rank = block_exclusive_scan(c, s_warp, &total);
+        uint32_t rank = group_exclusive_scan(c, s_warp, &total, nt);
         for (uint32_t wi = my_lo; wi < my_hi && rank < r_hi; ++wi) {
             uint32_t m = pop_word(bits, wi, W.p_lo, W.p_hi);
             if (rank + __popc(m) <= r_lo) { rank += __popc(m); continue; }
@@ -997,24 +1058,23 @@ push_local_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__
                 ++rank;
             }
         }
-        __syncthreads();
+        group_sync(nt);
         const uint32_t nrows = r_hi - r_lo;
         // span of every row of the unit: [out_ptr[j] + woff[k], out_ptr[j] + woff[k + 1])
         const NetView& nv = *W.nv;
-        for (uint32_t r = threadIdx.x; r < nrows; r += NT) {
+        for (uint32_t r = threadIdx.x; r < nrows; r += nt) {
             const uint32_t j = s_rows[r];
             const uint32_t* wo = nv.woff + W.rb_k + static_cast<unsigned long long>(j - W.p_lo) * W.ka1;
             const uint32_t s0 = __ldg(wo), s1 = __ldg(wo + 1);
             s_start[r] = __ldg(nv.out_ptr + j) + s0;
             s_len[r] = s1 - s0;
         }
-        __syncthreads();
+        group_sync(nt);
         const uint32_t* col = nv.out_col;
         const void* wts = nv.out_w;
-        // RL lanes per row: 32 (a warp per row) or 16 (two rows per warp, for short spans)
         constexpr uint32_t kRows = 32 / RL;
         const uint32_t sl = lane % RL;
-        const uint32_t rstride = (NT / 32) * kRows;
+        const uint32_t rstride = (nt / 32) * kRows;
         for (uint32_t r = warp * kRows + lane / RL; r < nrows; r += rstride) {
             const unsigned long long e0 = s_start[r], e1 = e0 + s_len[r];
             // the next row of these lanes: pull its span into L2 while this row is summed
@@ -1047,9 +1107,92 @@ push_local_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__
                 }
             }
         }
-        __syncthreads();
+        group_sync(nt);
     }
-    if (cur != 0xFFFFFFFFu) local_flush<FIX>(W, acc);
+    if (cur != 0xFFFFFFFFu) local_flush<FIX>(W, acc, nt);
+}
+
+// The cross-population part of a busy step: warps take chunks of the spike list from a
+// counter (the next chunk's number is fetched while the current one is worked on); the
+// chunk's row bounds are loaded side by side by its first lanes, so a chunk waits once for
+// them instead of once per row.  RL lanes per row.
+template <int ACC, int WT, int RL>
+__device__ __forceinline__ void push_cross(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets,
+                                           const SpikeList& sl, uint32_t count, const LocalPlan& lp) {
+    const uint32_t* rows_of = lp.scratch;
+    const uint32_t* win_prefix = lp.win_prefix;
+    uint32_t* counter = lp.scratch + 2 * lp.windows + 2;
+    constexpr uint32_t kRows = 32 / RL;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warps = gridDim.x * (kWindowThreads / 32);
+    // Rows next to each other in the list come from one population, and a small population's
+    // rows can carry ten times the mean cross-population degree (chunks of neighbours left one
+    // CTA working 160 us after the others on the 250k-neuron regional network).  So position r
+    // stands for list entry (r mod kDeal) x stride + r / kDeal, and chunks shrink towards the end
+    // of the list, to whole groups of kRows.
+    constexpr uint32_t kDeal = 64;
+    const uint32_t stride = (count + kDeal - 1) / kDeal, positions = stride * kDeal;
+    const unsigned long long keep = l2_policy_keep();
+    auto chunk_at = [&](uint32_t r) {
+        const uint32_t left = r < positions ? positions - r : 0u;
+        return max(kRows, min(kCrossChunk, left / (2u * warps)) / kRows * kRows);
+    };
+    uint32_t size = chunk_at(0), next = 0;
+    if (lane == 0) next = atomicAdd(counter, size);
+    for (;;) {
+        const uint32_t r0 = __shfl_sync(0xffffffffu, next, 0), m = size;
+        if (r0 >= positions) break;
+        size = chunk_at(r0 + warps * m);
+        if (lane == 0) next = atomicAdd(counter, size);
+        const uint32_t entry = ((r0 + lane) % kDeal) * stride + (r0 + lane) / kDeal;
+        unsigned long long beg = 0, beg2 = 0;
+        uint32_t len1 = 0, len = 0, net = 0;
+        if (lane < m && r0 + lane < positions && entry < count) {
+            const uint32_t v = __ldg(sl.list + entry);
+            net = n_nets > 1 ? find_net(vbase, n_nets, v) : 0u;
+            const NetView& nv = nets[net];
+            const uint32_t j = v - __ldg(vbase + net);
+            beg = __ldg(nv.out_ptr + j);
+            const unsigned long long end = __ldg(nv.out_ptr + j + 1);
+            len1 = static_cast<uint32_t>(end - beg);
+            beg2 = end;
+            if (nv.own_seg) {
+                const uint2 o = __ldg(nv.own_seg + j);
+                uint32_t p = __ldg(nv.tile_pop + j / kLifTile);
+                while (p + 1 < nv.n_pops && __ldg(nv.pop_off + p + 1) <= j) ++p;
+                if (o.x != o.y && rows_of[__ldg(win_prefix + net) + __ldg(nv.pop_win + p).x]) {
+                    len1 = o.x;                        // the windows take the own-population span
+                    beg2 = beg + o.y;
+                }
+            }
+            len = len1 + static_cast<uint32_t>(end - beg2);
+        }
+        for (uint32_t q = 0; q < m; q += kRows) {
+            const uint32_t src = q + lane / RL;          // lanes past m hold empty rows
+            const unsigned long long b = __shfl_sync(0xffffffffu, beg, src), b2 = __shfl_sync(0xffffffffu, beg2, src);
+            const uint32_t l1 = __shfl_sync(0xffffffffu, len1, src), ln = __shfl_sync(0xffffffffu, len, src);
+            const NetView& nv = nets[__shfl_sync(0xffffffffu, net, src)];
+            push_span<ACC, WT, 8, RL, true>(nv.out_col, nv.out_w, push_dst<ACC>(nv), b, l1, b2, ln, lane % RL, RL * 8u, keep);
+        }
+    }
+}
+
+template <int ACC, int WT, int RLW, int RLC>
+__global__ void __launch_bounds__(kWindowThreads, 1)
+push_window_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets, LocalPlan lp,
+                   uint32_t win_threads, SpikeList sl) {
+    extern __shared__ __align__(16) int acc[];
+    __shared__ uint32_t s_warp[33];
+    __shared__ uint32_t s_unit;
+    const uint32_t count = *sl.published;
+    const uint32_t total_units = lp.scratch[2 * lp.windows];
+    if (total_units == 0) {
+        push_rows<ACC, WT, 8, 32>(nets, vbase, n_nets, sl, count);
+    } else {
+        if (threadIdx.x < win_threads)
+            push_windows<WT, RLW, ACC == ACC_FIXED>(nets, lp, n_nets, total_units, acc, s_warp, &s_unit, win_threads);
+        push_cross<ACC, WT, RLC>(nets, vbase, n_nets, sl, count, lp);
+    }
 }
 
 __device__ inline uint32_t row_lower_bound(const uint32_t* __restrict__ col, unsigned long long beg,
@@ -1162,7 +1305,7 @@ push_tma_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ v
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncwarp();
-    const uint32_t count = *sl.count;
+    const uint32_t count = *sl.published;
     const uint32_t nw = gridDim.x * kTmaWarps;
     const unsigned long long keep = l2_policy_keep();
     // producer cursor (lane-uniform): list index, remaining range of the row, its network
@@ -1250,15 +1393,6 @@ push_tma_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ v
         if (lane == 0) atomicOr(&nets[0].clock->err, kErrTimeout);
         // let the other copy in flight land before the CTA's shared memory is released
         if (s_full[st ^ 1]) mbar_wait_bounded(&bars[st ^ 1], phase[st ^ 1]);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(sl.ticket, 1u) == gridDim.x - 1) {
-            *sl.count = 0u;
-            *sl.ticket = 0u;
-            __threadfence();
-        }
     }
 }
 
@@ -1403,7 +1537,7 @@ lif_pull_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ t
         bits[base >> 5] = wprop;
         if (record) nv.rec_bits[static_cast<size_t>(row) * nv.n_words + (base >> 5)] = wact;
     }
-    const unsigned long long ev = warp_sum_ull(sp ? static_cast<unsigned long long>(__ldg(nv.out_deg + i)) : 0ull);
+    const unsigned long long ev = warp_sum_ull(sp ? __ldg(nv.out_deg + i) : 0u);
     if (lane == 0 && ev) atomicAdd(&s_events, ev);
     if (stats) {
         const bool inc = valid && !excluded(nv, i);
@@ -1622,57 +1756,38 @@ cudaError_t launch_lif(const LaunchBatch& b, int jmode, uint32_t flags, int prop
     const uint32_t chunk = std::max(1u, b.lif_chunk);
     const dim3 grid(std::min((T + chunk - 1) / chunk, b.lif_ctas)), block(kLifThreads);
     switch (jmode) {
-        case J_DIRECT: lif_kernel<J_DIRECT><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk); break;
-        case J_FOLD: lif_kernel<J_FOLD><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk); break;
-        case J_FIXF: lif_kernel<J_FIXF><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk); break;
-        default: lif_kernel<J_ASIS><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk); break;
+        case J_DIRECT: lif_kernel<J_DIRECT><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
+        case J_FOLD: lif_kernel<J_FOLD><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
+        case J_FIXF: lif_kernel<J_FIXF><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
+        default: lif_kernel<J_ASIS><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
     }
     return cudaGetLastError();
 }
 
+// Threads of a CTA that take window units in a busy step of a PUSH_LOCAL form; the others
+// start on the cross-population rows.
+static uint32_t window_threads(const PushCfg& cfg) {
+    switch (cfg.param) {
+        case kLocalConcurrent: case kLocalConcurrentHalf: return 768;
+        case kLocalConcurrent2: return 512;
+        default: return kWindowThreads;
+    }
+}
+
+// The window kernel of a PUSH_LOCAL form: half-warp rows in the window sums (short spans) or in
+// the cross-population part (short rows).
+template <int ACC, int WT>
+static auto window_kernel(const PushCfg& cfg) {
+    return cfg.param == kLocalConcurrentHalf ? push_window_kernel<ACC, WT, 16, 32>
+         : cfg.lpr == 16 ? push_window_kernel<ACC, WT, 32, 16> : push_window_kernel<ACC, WT, 32, 32>;
+}
+
 template <int ACC, int WT>
 static cudaError_t push_launch_wt(const LaunchBatch& b, const PushCfg& cfg, uint32_t ctas, cudaStream_t s) {
-    constexpr bool FIX = ACC == ACC_FIXED;
-    if (cfg.kind == PUSH_LOCAL && ACC != ACC_EXACT &&
-        (cfg.param == kLocalConcurrent || cfg.param == kLocalConcurrent2 || cfg.param == kLocalConcurrentHalf) &&
-        b.aux && b.windows_total) {
-        // cross-population spans on the auxiliary stream, one (two) 256-thread CTA(s) per SM, next
-        // to the window kernel's 768 (512)-thread CTA: L2 reductions and shared-memory sums overlap
-        const bool two = cfg.param == kLocalConcurrent2;
-        cudaError_t e = cudaEventRecord(b.ev_fork, s);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(b.aux, b.ev_fork, 0);
-        if (e != cudaSuccess) return e;
-        if (two)
-            push_kernel_cross64<ACC, WT><<<b.sm_count * 2u, kPushThreads, 0, b.aux>>>(b.nets, b.vbase, b.n_nets, b.spikes);
-        else
-            push_kernel<ACC, WT, 8, 32, 1><<<b.sm_count, kPushThreads, 0, b.aux>>>(b.nets, b.vbase, b.n_nets, b.spikes);
-        e = cudaEventRecord(b.ev_join, b.aux);
-        if (e != cudaSuccess) return e;
-        local_prep_kernel<<<b.windows_total, 256, 0, s>>>(b.nets, b.win_prefix, b.n_nets, b.windows_total, b.local_scratch);
-        if (two)
-            push_local_kernel<WT, kLocalThreadsShared2, 32, FIX><<<b.sm_count, kLocalThreadsShared2, kLocalSmem, s>>>(
-                b.nets, b.win_prefix, b.n_nets, b.windows_total, b.local_scratch);
-        else if (cfg.param == kLocalConcurrentHalf)
-            push_local_kernel<WT, kLocalThreadsShared, 16, FIX><<<b.sm_count, kLocalThreadsShared, kLocalSmem, s>>>(
-                b.nets, b.win_prefix, b.n_nets, b.windows_total, b.local_scratch);
-        else
-            push_local_kernel<WT, kLocalThreadsShared, 32, FIX><<<b.sm_count, kLocalThreadsShared, kLocalSmem, s>>>(
-                b.nets, b.win_prefix, b.n_nets, b.windows_total, b.local_scratch);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b.ev_join, 0);
-        return e;
-    }
-    if (cfg.kind == PUSH_LOCAL && ACC != ACC_EXACT) {
-        const dim3 grid(ctas), block(kPushThreads);
-        if (cfg.lpr == 16)
-            push_kernel<ACC, WT, 8, 16, 1><<<grid, block, 0, s>>>(b.nets, b.vbase, b.n_nets, b.spikes);
-        else
-            push_kernel<ACC, WT, 8, 32, 1><<<grid, block, 0, s>>>(b.nets, b.vbase, b.n_nets, b.spikes);
-        if (b.windows_total) {
-            local_prep_kernel<<<b.windows_total, 256, 0, s>>>(b.nets, b.win_prefix, b.n_nets, b.windows_total, b.local_scratch);
-            push_local_kernel<WT, kLocalThreads, 32, FIX><<<b.sm_count, kLocalThreads, kLocalSmem, s>>>(
-                b.nets, b.win_prefix, b.n_nets, b.windows_total, b.local_scratch);
-        }
+    if (cfg.kind == PUSH_LOCAL && ACC != ACC_EXACT && b.local.windows) {
+        if constexpr (ACC != ACC_EXACT)
+            window_kernel<ACC, WT>(cfg)<<<b.sm_count, kWindowThreads, kLocalSmem, s>>>(b.nets, b.vbase, b.n_nets, b.local,
+                                                                                       window_threads(cfg), b.spikes);
     } else if (cfg.kind == PUSH_REG || cfg.kind == PUSH_LOCAL) {
         const dim3 grid(ctas), block(kPushThreads);
         if (cfg.lpr == 16) {
@@ -1704,19 +1819,11 @@ static cudaError_t push_prepare_wt(const PushCfg& cfg, int sm_count, uint32_t* c
     int per_sm = 0;
     cudaError_t e = cudaSuccess;
     if (cfg.kind == PUSH_LOCAL && ACC != ACC_EXACT) {
-        constexpr bool FIX = ACC == ACC_FIXED;
-        for (auto fn : {push_local_kernel<WT, kLocalThreads, 32, FIX>, push_local_kernel<WT, kLocalThreadsShared, 32, FIX>,
-                        push_local_kernel<WT, kLocalThreadsShared2, 32, FIX>, push_local_kernel<WT, kLocalThreadsShared, 16, FIX>})
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLocalSmem));
-        // the cross-population CTAs land on an SM first: ask for the largest shared-memory
-        // carve-out so a window CTA (229 KB) can join them there
-        for (auto fn : {push_kernel<ACC, WT, 8, 32, 1>, push_kernel<ACC, WT, 8, 16, 1>, push_kernel_cross64<ACC, WT>})
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         static_cast<int>(cudaSharedmemCarveoutMaxShared));
+        if constexpr (ACC != ACC_EXACT)
+            e = cudaFuncSetAttribute(window_kernel<ACC, WT>(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLocalSmem));
+        // the same form without windows falls back to push_kernel's register-staged rows
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cfg.lpr == 16 ? push_kernel<ACC, WT, 8, 16, 1> : push_kernel<ACC, WT, 8, 32, 1>,
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cfg.lpr == 16 ? push_kernel<ACC, WT, 8, 16> : push_kernel<ACC, WT, 8, 32>,
                                                               kPushThreads, 0);
     } else if (cfg.kind == PUSH_REG || cfg.kind == PUSH_LOCAL) {
         if (cfg.lpr == 16) {

@@ -8,6 +8,30 @@
 
 namespace dtb {
 
+// Windows of the population-window push over a batch.
+struct LocalPlan {
+    const uint32_t* win_prefix;   // device [n_nets + 1] cumulative windows
+    uint32_t windows;
+    uint32_t dense_min;           // spikes from which a step takes the windows
+    uint32_t always;              // 1: every population with a spike takes its windows
+    uint32_t unit_target;         // work units wanted in a busy step (a few per SM)
+    uint32_t flush_reds;          // reductions a window neuron costs to flush: 1 (float), 2 (fixed)
+    uint32_t* scratch;            // device [local_scratch_words(windows)], see local_prep
+};
+inline size_t local_scratch_words(size_t windows) { return 2 * windows + 4; }
+constexpr uint32_t kUnitsPerSm = 4;
+
+// Events (spikes x mean out-degree) from which a step takes the windows.  Scattered rows run at
+// 6.0 to 6.5 ps per event; the windows cost about 3.5 ps and 40 to 60 us of preparation, unit
+// start-up and uneven ends.  Measured, windows against scatter: 86 / 41 us at 6.0e6 events (250k
+// neurons, BF16, fixed), 84 / 82 us at 1.3e7, 110 / 118 us at 1.9e7 (200k, FP32, float),
+// 158 / 217 us at 3.2e7.
+constexpr uint64_t kDenseEvents = 16000000;
+inline uint32_t dense_min_spikes(uint64_t edges, uint64_t neurons) {
+    const uint64_t c = edges ? kDenseEvents * neurons / edges : 1u;
+    return static_cast<uint32_t>(c < 1 ? 1 : c > 0x7fffffffu ? 0x7fffffffu : c);
+}
+
 // One launch group: a batch of networks advanced together.
 struct LaunchBatch {
     const NetView* nets;          // device array [n_nets]
@@ -21,12 +45,8 @@ struct LaunchBatch {
     uint32_t push_ctas;
     uint32_t lif_ctas;            // persistent grid of the LIF kernel
     uint32_t lif_chunk;           // consecutive tiles a LIF CTA steps before striding (0 or 1: one)
-    const uint32_t* win_prefix;   // device [n_nets + 1] cumulative local-push windows
-    uint32_t windows_total;
-    uint32_t* local_scratch;      // device [2 * windows_total + 3]: rows per window, unit prefix, unit counter, ticket
+    LocalPlan local;              // population-window push (windows 0: none)
     uint32_t sm_count;
-    cudaStream_t aux;             // second stream of the concurrent local push (fork/join by events)
-    cudaEvent_t ev_fork, ev_join;
     SpikeList spikes;
 };
 
@@ -36,27 +56,25 @@ enum PushKind : int { PUSH_REG = 0, PUSH_TMA = 1, PUSH_LOCAL = 2 };
 struct PushCfg {
     int kind;    // PUSH_REG: register-staged loads, param = synapses in flight per lane (4, 8, 16)
                  // PUSH_TMA: bulk-copy staged rows, param = synapses per stage (256, 512)
-                 // PUSH_LOCAL: own-population synapses summed per window in shared memory,
-                 //   the rest register-staged (param = synapses in flight per lane, 8)
+                 // PUSH_LOCAL: in busy steps own-population synapses are summed per window in shared
+                 //   memory and the rest scattered; quiet steps scatter whole rows
     int param;
     int lpr = 32;  // PUSH_REG: lanes per row (32, 16, 8; sub-warp rows use 8 in flight per lane)
 };
 
 // Every variant the autotuner times.
 constexpr int kPushCandidates = 12;
-constexpr int kLocalConcurrent = 2008;   // PUSH_LOCAL param: cross-population part on a second stream
-constexpr int kLocalConcurrent2 = 2016;  // ... with two push CTAs per SM beside a 512-thread window CTA
-constexpr int kLocalConcurrentHalf = 3008;  // ... as 2008 with half-warp rows in the window kernel (short spans)
+// PUSH_LOCAL params: 8 (and 8 with 16 lanes per cross-population row) give every warp to the
+// windows first; the others start some of each CTA's warps on the cross-population rows at once
+constexpr int kLocalConcurrent = 2008;   // 24 warps on the windows, 8 on the cross-population rows
+constexpr int kLocalConcurrent2 = 2016;  // 16 and 16
+constexpr int kLocalConcurrentHalf = 3008;  // as 2008 with half-warp rows in the windows (short spans)
 extern const PushCfg kPushCands[kPushCandidates];
 // Sets kernel attributes and returns the persistent grid (max resident CTAs).
 // `acc` is the AccMode of the launch (float, exact or fixed-point accumulators).
 cudaError_t push_prepare(int acc, int weight_type, const PushCfg& cfg, int sm_count, uint32_t* ctas);
 cudaError_t launch_push(const LaunchBatch& b, int acc, int weight_type, const PushCfg& cfg, uint32_t ctas,
                         cudaStream_t s);
-// Kernels launch_push issues beyond the first (the local variant's prep and window passes).
-inline uint32_t push_extra_launches(const LaunchBatch& b, int acc, const PushCfg& cfg) {
-    return (cfg.kind == PUSH_LOCAL && acc != ACC_EXACT && b.windows_total) ? 2u : 0u;   // concurrent form: same count
-}
 cudaError_t launch_pull(const LaunchBatch& b, int gather, int weight_type, uint32_t flags, int prop_mode, cudaStream_t s);
 cudaError_t launch_fold_finish(const LaunchBatch& b, int acc, cudaStream_t s);
 // Per-population sums of the end-of-step synaptic currents (after the push of

@@ -231,8 +231,9 @@ int32_t dtb_info(void* engine, dtb_engine_info* info);
  * staged rows, param 256/512 synapses per stage) or 2 (population-local: each
  * row's own-population synapses are summed per window of its population in
  * shared memory, the rest as kind 0; param 8 or 1016, or 2008 / 2016 / 3008 for
- * the forms that run the rest on a second stream beside the window kernel; float
- * push mode only, the exact mode runs kind 0 instead);
+ * the forms that start some warps of each CTA on the rest at once; not in the
+ * exact mode, which runs kind 0 instead).  A form chosen here takes the windows in
+ * every step; chosen by the tuner it takes them in steps of many events only.
  * kind < 0 re-enables the autotuner.  From step 300 it reads the spike count of
  * every step for 50 steps, then times every variant on the live spike lists of
  * four steps with at least half the peak count seen (and 0.2 % of the neurons),

@@ -1,0 +1,60 @@
+"""The population-window push decides per step: a step of few events scatters whole rows, a busy
+one sums own-population spans in windows and scatters the rest, population by population.  With
+the fixed-point push every route gives the same integer sums, so a run in which the tuner's
+window form crosses the threshold equals the register push bit for bit; so do single steps of few
+rows, whose rows are cut into parts."""
+import numpy as np
+import pytest
+
+from dtb_b200 import engine as E
+from dtb_b200 import network as nw
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(spec, variant, steps, wt, chunk=100):
+    with E.Engine.structured(spec, weight_type=wt, seed=9) as eng:
+        if variant is not None:
+            eng.set_push_variant(*variant)
+        freqs, events = [], 0
+        for _ in range(steps // chunk):
+            r = eng.run(chunk, syn_mode=E.SYN_PUSH_FIXED)
+            freqs.append(r.freqs)
+            events += r.events
+        return np.concatenate(freqs), events, eng.read_state(E.STATE_V), eng.read_state(E.STATE_J), eng.info()
+
+
+@pytest.mark.parametrize("n,pops,degree,wt", [(60_011, 7, 600, E.W_F32), (90_000, 40, 400, E.W_BF16)])
+def test_tuned_window_form_gives_the_register_pushs_bits(gpu, n, pops, degree, wt):
+    spec = nw.structured_spec(n, pops, degree, seed=31)
+    f0, e0, v0, j0, _ = _run(spec, (E.PUSH_REG, 8), 1000, wt)
+    f1, e1, v1, j1, inf = _run(spec, None, 1000, wt)              # autotuned
+    f2, e2, v2, j2, _ = _run(spec, (E.PUSH_LOCAL, 2016), 1000, wt)   # windows in every step
+    assert f0.sum(1).max() > 0.1 * n and np.median(f0.sum(1)) < 0.01 * n     # quiet steps and bursts
+    for f, e, v, j in ((f1, e1, v1, j1), (f2, e2, v2, j2)):
+        assert np.array_equal(f0, f) and e0 == e
+        assert np.array_equal(v0, v) and np.array_equal(j0, j)
+
+
+@pytest.mark.parametrize("out_degree", [1, 255, 256, 257, 2047, 2049, 5000])
+def test_few_long_rows_are_cut_into_parts(gpu, out_degree):
+    """A step whose only spikes are three neurons of a given out-degree (a strong drive on them
+    alone): J must hold every one of their synapses once."""
+    n = 6000
+    rng = np.random.default_rng(out_degree)
+    src = np.array([5, 3001, 5999])
+    pre = np.repeat(src, out_degree).astype(np.uint32)
+    post = rng.integers(0, n, pre.size).astype(np.uint32)
+    w = (rng.integers(0, 256, (pre.size, 2)) / 256.0).astype(np.float32)
+    kind = rng.integers(0, 2, pre.size).astype(np.uint8)
+    prop = nw.lif_property(n, 0)
+    prop[src, 2] = 1e5                       # I_ext: over threshold in the first step
+    net = dict(property=prop, input_neuron_idx=pre, output_neuron_idx=post, input_channel_offset=kind, weight=w)
+    ref = np.zeros((n, 4))
+    for k in (0, 1):
+        np.add.at(ref, (post, 2 * kind.astype(int) + k), w[:, k].astype(np.float64))
+    for syn in (E.SYN_PUSH, E.SYN_PUSH_FIXED, E.SYN_PUSH_EXACT):
+        with E.Engine.from_arrays(net) as eng:
+            r = eng.run(1, use_ou=False, syn_mode=syn)
+            assert r.freqs.sum() == 3 and r.events == pre.size
+            assert np.array_equal(eng.read_state(E.STATE_J), ref.astype(np.float32))    # dyadic weights: exact in any order
