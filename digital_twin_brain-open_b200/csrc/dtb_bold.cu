@@ -22,35 +22,100 @@ struct BoldConst {
     float one_m_e0, div_alpha, div_alpha_m1, seven_e0, e0_term;
 };
 
-__global__ void __launch_bounds__(128)
-bold_kernel(BoldConst c, uint32_t n, uint32_t steps, const float* __restrict__ u, float* __restrict__ state,
+// Steps taken together.  A step is four recurrences of very different weight: (s, f_in) needs
+// two divisions, v a power, q two powers and three divisions, and only v's and q's last
+// operations wait for the step before.  One warp per scheduler is all a DA window fills (23,000
+// voxels are 719 warps for 592 schedulers), so a step-by-step loop waits for each power in turn;
+// kBoldSteps steps side by side keep that many of them in flight.
+constexpr int kBoldSteps = 4;
+constexpr int kBoldThreads = 64;    // small blocks spread a window's few warps evenly over the SMs
+constexpr int kBoldMostWhole = 16;  // largest 1/alpha taken by squaring
+
+// x^n by squaring for the whole exponent n >= 1 (uniform over the grid).
+__device__ __forceinline__ float pow_whole(float x, int n) {
+    float r = 1.0f, b = x;
+    bool first = true;
+    for (; n; n >>= 1) {
+        if (n & 1) {
+            r = first ? b : __fmul_rn(r, b);
+            first = false;
+        }
+        if (n > 1) b = __fmul_rn(b, b);
+    }
+    return r;
+}
+
+// v^(1/alpha - 1) and v^(1/alpha).  WHOLE: 1/alpha is the whole number `whole` (5 for the default
+// alpha of 0.2); the powers are then products of at most a few roundings, within the error of
+// powf, and off the critical path's ~100 instructions each.
+template <bool WHOLE>
+__device__ __forceinline__ void bold_powers(const BoldConst& c, int whole, float v, float& pm1, float& p) {
+    if constexpr (WHOLE) {
+        pm1 = whole > 1 ? pow_whole(v, whole - 1) : 1.0f;
+        p = whole > 1 ? __fmul_rn(pm1, v) : v;
+    } else {
+        pm1 = powf(v, c.div_alpha_m1);
+        p = powf(v, c.div_alpha);
+    }
+}
+
+// N steps from step k on.
+template <bool WHOLE, int N>
+__device__ __forceinline__ void bold_steps(const BoldConst& c, int whole, uint32_t n, uint32_t i, uint32_t k,
+                                           const float* __restrict__ u, float* __restrict__ out, float& s, float& q, float& v,
+                                           float& f) {
+    float uk[N], fk[N], fq[N], pm1[N], vn[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) uk[j] = __ldcs(u + static_cast<size_t>(k + j) * n + i);
+    // s and f_in: d_s = epsilon * u - s / tao_s - (f_in - 1) / tao_f
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        fk[j] = f;
+        const float d_s = __fsub_rn(__fsub_rn(__fmul_rn(c.eps, uk[j]), __fdiv_rn(s, c.tao_s)),
+                                    __fdiv_rn(__fsub_rn(f, 1.0f), c.tao_f));
+        f = __fadd_rn(f, __fmul_rn(s, c.dt));
+        f = f > 0.0f ? f : 0.0f;
+        s = __fadd_rn(s, __fmul_rn(d_s, c.dt));
+    }
+    // f_in * q_part / E_0, q_part = 1 - (1 - E_0) ** (1 / f_in) where f_in > 0, else 1
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const float part = fk[j] > 0.0f ? __fsub_rn(1.0f, powf(c.one_m_e0, __fdiv_rn(1.0f, fk[j]))) : 1.0f;
+        fq[j] = __fdiv_rn(__fmul_rn(fk[j], part), c.e0);
+    }
+    // v, with the power that q takes of its old value
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        float p;
+        bold_powers<WHOLE>(c, whole, v, pm1[j], p);
+        const float dv = __fdiv_rn(__fsub_rn(fk[j], p), c.tao_0);
+        v = __fadd_rn(v, __fmul_rn(dv, c.dt));
+        vn[j] = v;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const float dq = __fdiv_rn(__fsub_rn(fq[j], __fmul_rn(q, pm1[j])), c.tao_0);
+        q = __fadd_rn(q, __fmul_rn(dq, c.dt));
+        if (out) {
+            // V_0 * (7 E_0 (1 - q) + 2 (1 - q / v) + (2 E_0 - 0.2) (1 - v))
+            const float a = __fmul_rn(c.seven_e0, __fsub_rn(1.0f, q));
+            const float b = __fmul_rn(2.0f, __fsub_rn(1.0f, __fdiv_rn(q, vn[j])));
+            const float d = __fmul_rn(c.e0_term, __fsub_rn(1.0f, vn[j]));
+            out[static_cast<size_t>(k + j) * n + i] = __fmul_rn(c.v0, __fadd_rn(__fadd_rn(a, b), d));
+        }
+    }
+}
+
+template <bool WHOLE>
+__global__ void __launch_bounds__(kBoldThreads)
+bold_kernel(BoldConst c, int whole, uint32_t n, uint32_t steps, const float* __restrict__ u, float* __restrict__ state,
             float* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = state[i], q = state[n + i], v = state[2 * n + i], f = state[3 * n + i];
-    for (uint32_t k = 0; k < steps; ++k) {
-        const float uk = __ldcs(u + static_cast<size_t>(k) * n + i);
-        // d_s = epsilon * u - s / tao_s - (f_in - 1) / tao_f
-        const float d_s = __fsub_rn(__fsub_rn(__fmul_rn(c.eps, uk), __fdiv_rn(s, c.tao_s)),
-                                    __fdiv_rn(__fsub_rn(f, 1.0f), c.tao_f));
-        // q_part = 1 - (1 - E_0) ** (1 / f_in) where f_in > 0, else 1
-        const float q_part = f > 0.0f ? __fsub_rn(1.0f, powf(c.one_m_e0, __fdiv_rn(1.0f, f))) : 1.0f;
-        const float dq = __fdiv_rn(__fsub_rn(__fdiv_rn(__fmul_rn(f, q_part), c.e0), __fmul_rn(q, powf(v, c.div_alpha_m1))),
-                                   c.tao_0);
-        q = __fadd_rn(q, __fmul_rn(dq, c.dt));
-        const float dv = __fdiv_rn(__fsub_rn(f, powf(v, c.div_alpha)), c.tao_0);
-        v = __fadd_rn(v, __fmul_rn(dv, c.dt));
-        f = __fadd_rn(f, __fmul_rn(s, c.dt));
-        f = f > 0.0f ? f : 0.0f;
-        s = __fadd_rn(s, __fmul_rn(d_s, c.dt));
-        if (out) {
-            // V_0 * (7 E_0 (1 - q) + 2 (1 - q / v) + (2 E_0 - 0.2) (1 - v))
-            const float a = __fmul_rn(c.seven_e0, __fsub_rn(1.0f, q));
-            const float b = __fmul_rn(2.0f, __fsub_rn(1.0f, __fdiv_rn(q, v)));
-            const float d = __fmul_rn(c.e0_term, __fsub_rn(1.0f, v));
-            out[static_cast<size_t>(k) * n + i] = __fmul_rn(c.v0, __fadd_rn(__fadd_rn(a, b), d));
-        }
-    }
+    uint32_t k = 0;
+    for (; k + kBoldSteps <= steps; k += kBoldSteps) bold_steps<WHOLE, kBoldSteps>(c, whole, n, i, k, u, out, s, q, v, f);
+    for (; k < steps; ++k) bold_steps<WHOLE, 1>(c, whole, n, i, k, u, out, s, q, v, f);
     state[i] = s;
     state[n + i] = q;
     state[2 * n + i] = v;
@@ -80,7 +145,14 @@ int32_t dtb_bold_run(const dtb_bold_params* p, uint32_t n, uint32_t steps, const
                            static_cast<float>(div_alpha), static_cast<float>(div_alpha - 1.0),
                            static_cast<float>(7.0 * p->E_0), static_cast<float>(2.0 * p->E_0 - 0.2)};
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    dtb::bold_kernel<<<(n + 127) / 128, 128, 0, s>>>(c, n, steps, u, state, out);
+    // 1 / alpha as float32: a small whole number takes the products
+    const bool whole = c.div_alpha >= 1.0f && c.div_alpha <= dtb::kBoldMostWhole && c.div_alpha == std::floor(c.div_alpha) &&
+                       c.div_alpha_m1 == c.div_alpha - 1.0f;
+    const uint32_t blocks = (n + dtb::kBoldThreads - 1) / dtb::kBoldThreads;
+    if (whole)
+        dtb::bold_kernel<true><<<blocks, dtb::kBoldThreads, 0, s>>>(c, static_cast<int>(c.div_alpha), n, steps, u, state, out);
+    else
+        dtb::bold_kernel<false><<<blocks, dtb::kBoldThreads, 0, s>>>(c, 0, n, steps, u, state, out);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return dtb::cuda_fail(e, "bold_kernel");
     return DTB_OK;
