@@ -9,87 +9,158 @@
 // I[e,v] = y[v] + sqrt(sigma) n[e,v] - w_hat[e,v,S-1]:
 //   w = w_hat + rate * I[e,v] * sum_e' T[e',v] d[e',v,s]
 //             + (1 - rate) * sum_e' G[e,e'] d[e',v,s],   G = I T^T / V.
-// Three kernels: per-voxel statistics (one warp per voxel), the E x E gain G,
-// and the update (one thread per output).  Everything accumulates in double and
-// is rounded once, so the result is the float32 rounding of the exact update
-// (the reference's float32 reductions and GEMMs agree to ~1e-7 relative).
+// Three kernels: per-voxel statistics, the E x E gain G, and the update.  Everything
+// accumulates in double and is rounded once, so the result is the float32 rounding of the
+// exact update (the reference's float32 reductions and GEMMs agree to ~1e-7 relative).
+#include <algorithm>
+
 #include "dtb_engine.h"
 
 namespace dtb {
 
-__global__ void __launch_bounds__(256)
-da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, const float* __restrict__ w, const float* __restrict__ y,
-                const float* __restrict__ noise, double sigma, double* __restrict__ mean, double* __restrict__ temp,
-                double* __restrict__ innov, double* __restrict__ colsum) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+constexpr int kDaThreads = 256;
+
+// Statistics: a CTA takes `vb` consecutive voxels, whose vb x S columns are contiguous in every
+// member's row, so the members' loads are coalesced (one warp per voxel read 4 bytes of 32
+// different lines per load).  The 256 threads are `groups` rows of `width` lanes (width a power
+// of two, at least vb x S where that fits); partial sums of a column meet in shared memory in a
+// fixed order.
+__global__ void __launch_bounds__(kDaThreads)
+da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, uint32_t vb, uint32_t width, const float* __restrict__ w,
+                const float* __restrict__ y, const float* __restrict__ noise, double sigma, double* __restrict__ mean,
+                double* __restrict__ temp, double* __restrict__ innov, double* __restrict__ colsum) {
+    __shared__ double s_part[kDaThreads];
+    const uint32_t groups = kDaThreads / width, g = threadIdx.x / width, x = threadIdx.x % width;
+    const uint32_t v0 = blockIdx.x * vb, nv = min(vb, V - v0), cols = nv * S;
+    const size_t row = static_cast<size_t>(V) * S;
     const double sq = sqrt(sigma);
-    for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < V; v += nw) {
-        for (uint32_t s = 0; s < S; ++s) {
-            double acc = 0.0;
-            for (uint32_t e = lane; e < E; e += 32) acc += w[(static_cast<size_t>(e) * V + v) * S + s];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) mean[static_cast<size_t>(v) * S + s] = acc / E;
+    // sum of a column's partial sums, for every thread of lane column x
+    auto meet = [&](double part) {
+        __syncthreads();
+        s_part[threadIdx.x] = part;
+        __syncthreads();
+        double sum = 0.0;
+        for (uint32_t k = 0; k < groups; ++k) sum += s_part[k * width + x];
+        return sum;
+    };
+    for (uint32_t c0 = 0; c0 < cols; c0 += width) {         // one pass unless S is wider than the CTA
+        const uint32_t col = c0 + x;
+        const bool in = col < cols;
+        const uint32_t vl = in ? col / S : 0u, v = v0 + vl;
+        const float* base = w + static_cast<size_t>(v0) * S + (in ? col : 0u);
+        double acc = 0.0;
+        if (in) {
+#pragma unroll 4
+            for (uint32_t e = g; e < E; e += groups) acc += base[e * row];
         }
-        __syncwarp();
-        const double ml = mean[static_cast<size_t>(v) * S + S - 1];
+        const double m = meet(acc) / E;
+        // the voxel's last column: its mean and variance
+        const float* last = w + static_cast<size_t>(v) * S + S - 1;
+        double al = 0.0;
+        if (in) {
+#pragma unroll 4
+            for (uint32_t e = g; e < E; e += groups) al += last[e * row];
+        }
+        const double ml = meet(al) / E;
         double cx = 0.0;
-        for (uint32_t e = lane; e < E; e += 32) {
-            const double d = w[(static_cast<size_t>(e) * V + v) * S + S - 1] - ml;
-            cx += d * d;
+        if (in) {
+#pragma unroll 4
+            for (uint32_t e = g; e < E; e += groups) {
+                const double d = last[e * row] - ml;
+                cx += d * d;
+            }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cx += __shfl_xor_sync(0xffffffffu, cx, o);
-        const double cxx = cx / (E - 1) + sigma;
-        for (uint32_t e = lane; e < E; e += 32) {
-            const double last = w[(static_cast<size_t>(e) * V + v) * S + S - 1];
-            temp[static_cast<size_t>(e) * V + v] = (last - ml) / cxx / (E - 1);
-            innov[static_cast<size_t>(e) * V + v] = static_cast<double>(y[v]) + sq * noise[static_cast<size_t>(e) * V + v] - last;
+        const double cxx = meet(cx) / (E - 1) + sigma;
+        double cs = 0.0;
+        if (in) {
+            const bool lead = col % S == S - 1;              // the lane that writes the voxel's temp and innov
+            for (uint32_t e = g; e < E; e += groups) {
+                const double l = last[e * row];
+                const double t = (l - ml) / cxx / (E - 1);
+                cs += t * (base[e * row] - m);
+                if (lead) {
+                    temp[static_cast<size_t>(e) * V + v] = t;
+                    innov[static_cast<size_t>(e) * V + v] = static_cast<double>(y[v]) + sq * noise[static_cast<size_t>(e) * V + v] - l;
+                }
+            }
         }
-        __syncwarp();
-        for (uint32_t s = 0; s < S; ++s) {
-            const double m = mean[static_cast<size_t>(v) * S + s];
-            double acc = 0.0;
-            for (uint32_t e = lane; e < E; e += 32)
-                acc += temp[static_cast<size_t>(e) * V + v] * (w[(static_cast<size_t>(e) * V + v) * S + s] - m);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) colsum[static_cast<size_t>(v) * S + s] = acc;
+        const double sum = meet(cs);
+        if (in && g == 0) {
+            mean[static_cast<size_t>(v0) * S + col] = m;
+            colsum[static_cast<size_t>(v0) * S + col] = sum;
         }
     }
 }
 
-// G[e][f] = sum_v I[e,v] T[f,v] / V: one warp per (e, f).
-__global__ void __launch_bounds__(256)
+// G[e][f] = sum_v I[e,v] T[f,v] / V.  A CTA makes an 8 x 8 tile: rows of 64 voxels of both
+// factors are staged in shared memory and four threads share a product's voxels (a warp per
+// product re-read both rows for each of the E^2 products).
+constexpr int kGainTile = 8, kGainVox = 64;
+__global__ void __launch_bounds__(kDaThreads)
 da_gain_kernel(uint32_t E, uint32_t V, const double* __restrict__ innov, const double* __restrict__ temp,
                double* __restrict__ gain) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < E * E; k += nw) {
-        const uint32_t e = k / E, f = k % E;
-        double acc = 0.0;
-        for (uint32_t v = lane; v < V; v += 32) acc += innov[static_cast<size_t>(e) * V + v] * temp[static_cast<size_t>(f) * V + v];
+    __shared__ double s_i[kGainTile][kGainVox + 1], s_t[kGainTile][kGainVox + 1];
+    const uint32_t tiles = (E + kGainTile - 1) / kGainTile;
+    const uint32_t e0 = blockIdx.x / tiles * kGainTile, f0 = blockIdx.x % tiles * kGainTile;
+    const uint32_t part = threadIdx.x & 3u, pair = threadIdx.x >> 2, e = pair / kGainTile, f = pair % kGainTile;
+    double acc = 0.0;
+    for (uint32_t v0 = 0; v0 < V; v0 += kGainVox) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < kGainTile * kGainVox; k += kDaThreads) {
+            const uint32_t r = k / kGainVox, v = v0 + k % kGainVox;
+            s_i[r][k % kGainVox] = v < V && e0 + r < E ? innov[static_cast<size_t>(e0 + r) * V + v] : 0.0;
+            s_t[r][k % kGainVox] = v < V && f0 + r < E ? temp[static_cast<size_t>(f0 + r) * V + v] : 0.0;
+        }
+        __syncthreads();
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) gain[k] = acc / V;
+        for (uint32_t k = part; k < kGainVox; k += 4) acc = __fma_rn(s_i[e][k], s_t[f][k], acc);
     }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    if (part == 0 && e0 + e < E && f0 + f < E) gain[static_cast<size_t>(e0 + e) * E + f0 + f] = acc / V;
 }
 
-__global__ void __launch_bounds__(256)
+// Update: a thread owns one column (voxel, state) for kUpdRows members, so a deviation is read
+// and widened once for kUpdRows products (one thread per output widened it for each); the
+// members' gains sit in shared memory and are read as broadcasts, kUpdChunk of them at a time.
+constexpr int kUpdThreads = 128, kUpdRows = 10, kUpdChunk = 128;
+__global__ void __launch_bounds__(kUpdThreads)
 da_update_kernel(uint32_t E, uint32_t V, uint32_t S, const float* __restrict__ w, const double* __restrict__ mean,
                  const double* __restrict__ innov, const double* __restrict__ colsum, const double* __restrict__ gain,
                  double rate, float* __restrict__ out) {
-    const size_t total = static_cast<size_t>(E) * V * S;
-    for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < total; k += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint32_t s = static_cast<uint32_t>(k % S);
-        const uint32_t v = static_cast<uint32_t>((k / S) % V);
-        const uint32_t e = static_cast<uint32_t>(k / (static_cast<size_t>(S) * V));
-        const size_t col = static_cast<size_t>(v) * S + s;
-        const double m = mean[col];
-        double acc = 0.0;
-        for (uint32_t f = 0; f < E; ++f) acc += gain[static_cast<size_t>(e) * E + f] * (w[static_cast<size_t>(f) * V * S + col] - m);
-        const double x = static_cast<double>(w[k]) + rate * innov[static_cast<size_t>(e) * V + v] * colsum[col] + (1.0 - rate) * acc;
+    __shared__ double s_gain[kUpdChunk][kUpdRows];
+    const size_t cols = static_cast<size_t>(V) * S;
+    const size_t col = static_cast<size_t>(blockIdx.x) * kUpdThreads + threadIdx.x;
+    const uint32_t e0 = blockIdx.y * kUpdRows;
+    const bool in = col < cols;
+    const double m = in ? mean[col] : 0.0;
+    double acc[kUpdRows] = {};
+    for (uint32_t f0 = 0; f0 < E; f0 += kUpdChunk) {
+        const uint32_t nf = min(static_cast<uint32_t>(kUpdChunk), E - f0);
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < nf * kUpdRows; k += kUpdThreads) {
+            const uint32_t r = k / nf, f = k % nf;
+            s_gain[f][r] = e0 + r < E ? gain[static_cast<size_t>(e0 + r) * E + f0 + f] : 0.0;
+        }
+        __syncthreads();
+        if (in) {
+#pragma unroll 4
+            for (uint32_t f = 0; f < nf; ++f) {
+                const double d = w[static_cast<size_t>(f0 + f) * cols + col] - m;
+#pragma unroll
+                for (int r = 0; r < kUpdRows; ++r) acc[r] = __fma_rn(s_gain[f][r], d, acc[r]);
+            }
+        }
+    }
+    if (!in) return;
+    const uint32_t v = static_cast<uint32_t>(col / S);
+    const double cs = colsum[col];
+#pragma unroll
+    for (int r = 0; r < kUpdRows; ++r) {
+        const uint32_t e = e0 + r;
+        if (e >= E) break;
+        const size_t k = static_cast<size_t>(e) * cols + col;
+        const double x = static_cast<double>(w[k]) + rate * innov[static_cast<size_t>(e) * V + v] * cs + (1.0 - rate) * acc[r];
         out[k] = static_cast<float>(x);
     }
 }
@@ -113,11 +184,16 @@ extern "C" int32_t dtb_da_filter(uint32_t ensembles, uint32_t voxels, uint32_t s
     double* temp = colsum + n_mean;
     double* innov = temp + n_ev;
     double* gain = innov + n_ev;
-    const uint32_t warps_v = static_cast<uint32_t>(std::min<size_t>((V + 7) / 8, 4096));
-    dtb::da_stats_kernel<<<warps_v, 256, 0, s>>>(ensembles, voxels, states, w_hat, bold_y, noise, bold_sigma, mean, temp, innov, colsum);
-    dtb::da_gain_kernel<<<static_cast<uint32_t>(std::min<size_t>((E * E + 7) / 8, 4096)), 256, 0, s>>>(ensembles, voxels, innov, temp, gain);
-    dtb::da_update_kernel<<<static_cast<uint32_t>(std::min<size_t>((E * V * S + 255) / 256, 65535)), 256, 0, s>>>(
-        ensembles, voxels, states, w_hat, mean, innov, colsum, gain, rate, w_out);
+    // voxels per statistics CTA: as many as fill its threads once over, down to one
+    const uint32_t vb = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(64 / S, V)));
+    uint32_t width = 1;
+    while (width < vb * S && width < dtb::kDaThreads) width *= 2;
+    dtb::da_stats_kernel<<<static_cast<uint32_t>((V + vb - 1) / vb), dtb::kDaThreads, 0, s>>>(
+        ensembles, voxels, states, vb, width, w_hat, bold_y, noise, bold_sigma, mean, temp, innov, colsum);
+    const uint32_t tiles = (ensembles + dtb::kGainTile - 1) / dtb::kGainTile;
+    dtb::da_gain_kernel<<<tiles * tiles, dtb::kDaThreads, 0, s>>>(ensembles, voxels, innov, temp, gain);
+    const dim3 grid(static_cast<uint32_t>((V * S + dtb::kUpdThreads - 1) / dtb::kUpdThreads), (ensembles + dtb::kUpdRows - 1) / dtb::kUpdRows);
+    dtb::da_update_kernel<<<grid, dtb::kUpdThreads, 0, s>>>(ensembles, voxels, states, w_hat, mean, innov, colsum, gain, rate, w_out);
     e = cudaGetLastError();
     cudaFreeAsync(buf, s);
     if (e != cudaSuccess) return dtb::cuda_fail(e, "dtb_da_filter");
