@@ -16,7 +16,13 @@ inline uint32_t compact_tiles(uint32_t n) {
     return static_cast<uint32_t>((static_cast<uint64_t>(n) + kCompactTileNeurons - 1) / kCompactTileNeurons);
 }
 
-// Count, scan and write; `tile_scratch` holds compact_tiles(n) words.
+// Bitmaps up to kDirectNeurons are compacted by one launch that re-reads its prefixes and uses
+// no scratch; the re-reads grow with the square of the size (128 MB from L2 at the limit, about
+// the time the two further launches of the tiled form take).
+constexpr int kDirectWords = 1024;
+constexpr uint32_t kDirectNeurons = 8u << 20;
+
+// Count, scan and write (tile_scratch unused up to kDirectNeurons); `tile_scratch` holds compact_tiles(n) words.
 cudaError_t compact_launch(const uint32_t* bits, uint32_t n, uint32_t* idx, uint32_t* count, uint32_t* tile_scratch,
                            cudaStream_t s);
 
