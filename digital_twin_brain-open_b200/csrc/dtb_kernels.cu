@@ -1399,47 +1399,163 @@ push_tma_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ v
 // ---------------------------------------------------------------------------
 // Deterministic in-degree gather of 32 neurons by one warp: lane k returns the
 // exact fixed-point input of neuron base + k (sum over in-edges whose source
-// spiked in `prev_bits`).
+// spiked in `prev_bits`, a bitmap in global or shared memory).  U edges are in
+// flight per lane; the warp's 64-bit sums are formed only for rows with a hit
+// (most steps of a bursting network hit few rows).
 // ---------------------------------------------------------------------------
-template <int WT>
-__device__ inline void gather32(const NetView& nv, uint32_t base, const uint32_t* __restrict__ prev_bits,
-                                int lane, long long acc_out[4]) {
+template <int WT, int U>
+__device__ __forceinline__ void gather32(const NetView& nv, uint32_t base, const uint32_t* prev_bits, int lane,
+                                         long long acc_out[4]) {
     acc_out[0] = acc_out[1] = acc_out[2] = acc_out[3] = 0;
     const uint32_t last = min(base + 32u, nv.n);
+    const uint32_t* __restrict__ in_col = nv.in_col;
+    // row bounds of the warp's neurons, one per lane
+    unsigned long long my_beg = 0, my_end = 0;
+    if (base + lane < last) {
+        my_beg = __ldg(nv.in_ptr + base + lane);
+        my_end = __ldg(nv.in_ptr + base + lane + 1);
+    }
     for (uint32_t j = base; j < last; ++j) {
-        const unsigned long long beg = __ldg(nv.in_ptr + j), end = __ldg(nv.in_ptr + j + 1);
+        const unsigned long long beg = __shfl_sync(0xffffffffu, my_beg, j - base), end = __shfl_sync(0xffffffffu, my_end, j - base);
         long long a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        for (unsigned long long e = beg + lane; e < end; e += 128) {
-            uint32_t c[4];
+        uint32_t any = 0;
+        for (unsigned long long e = beg + lane; e < end; e += 32ull * U) {
+            uint32_t c[U];
             uint32_t hit = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const unsigned long long idx = e + 32ull * q;
-                c[q] = idx < end ? __ldcs(nv.in_col + idx) : 0u;
-            }
+            for (int q = 0; q < U; ++q) c[q] = e + 32ull * q < end ? __ldcs(in_col + e + 32ull * q) : 0u;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const unsigned long long idx = e + 32ull * q;
-                if (idx < end) {
-                    const uint32_t src = c[q] & kIndexMask;
-                    hit |= ((__ldg(prev_bits + (src >> 5)) >> (src & 31u)) & 1u) << q;
-                }
+            for (int q = 0; q < U; ++q) {
+                const uint32_t src = c[q] & kIndexMask;
+                if (e + 32ull * q < end) hit |= ((prev_bits[src >> 5] >> (src & 31u)) & 1u) << q;
             }
+            any |= hit;
+            if (hit) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if ((hit >> q) & 1u) {
-                    const float2 w = load_weight<WT>(nv.in_w, e + 32ull * q);
-                    const long long f0 = float_to_fix(w.x), f1 = float_to_fix(w.y);
-                    if (c[q] >> 31) { a2 += f0; a3 += f1; } else { a0 += f0; a1 += f1; }
+                for (int q = 0; q < U; ++q) {
+                    if ((hit >> q) & 1u) {
+                        const float2 w = load_weight<WT>(nv.in_w, e + 32ull * q);
+                        const long long f0 = float_to_fix(w.x), f1 = float_to_fix(w.y);
+                        if (c[q] >> 31) { a2 += f0; a3 += f1; } else { a0 += f0; a1 += f1; }
+                    }
                 }
             }
         }
+        if (!__any_sync(0xffffffffu, any)) continue;
         a0 = warp_sum_ll(a0);
         a1 = warp_sum_ll(a1);
         a2 = warp_sum_ll(a2);
         a3 = warp_sum_ll(a3);
         if (static_cast<uint32_t>(lane) == j - base) {
             acc_out[0] = a0; acc_out[1] = a1; acc_out[2] = a2; acc_out[3] = a3;
+        }
+    }
+}
+
+// One pull step as the warps of a CTA see it.
+struct PullStep {
+    uint32_t flags;
+    int prop_mode;
+    float t;
+    unsigned long long n, inj_base;
+    long long row;
+    bool stats, record;
+};
+
+__device__ __forceinline__ PullStep pull_step(const NetView& nv, uint32_t flags, int prop_mode, uint32_t& err) {
+    PullStep ps{flags, prop_mode, __fadd_rn(nv.clock->t, nv.dt), nv.clock->n + 1, nv.clock->inj_base,
+                static_cast<long long>(nv.clock->n - nv.clock->run_base), (flags & kFlagStats) != 0,
+                (flags & kFlagRecord) != 0 && nv.rec_bits != nullptr};
+    if ((ps.stats || ps.record) && (ps.row < 0 || ps.row >= static_cast<long long>(nv.hist_cap))) {
+        ps.stats = false;
+        ps.record = false;
+        err |= kErrHistOverflow;
+    }
+    return ps;
+}
+
+// Gather (GATHER) and step the 32 neurons from `base` on; `prev` is the previous step's bitmap.
+template <int GATHER, int WT, int U>
+__device__ __forceinline__ void pull_step32(const NetView& nv, const PullStep& ps, uint32_t base, const uint32_t* prev, int lane,
+                                            const StatAcc& sa, unsigned long long* s_events, uint32_t& err) {
+    const uint32_t i = base + lane;
+    long long acc[4] = {0, 0, 0, 0};
+    if constexpr (GATHER) gather32<WT, U>(nv, base, prev, lane, acc);
+    const bool valid = i < nv.n;
+    bool active = false, sp = false;
+    float vnew = 0.f;
+    uint32_t p = 0;
+    if (valid) {
+        p = find_pop(nv.pop_off, nv.n_pops, i);
+        PopParams pp;
+        load_pop_params(nv, p, i, pp);
+        float4 Jv = nv.J[i];
+        float* Jc = reinterpret_cast<float*>(&Jv);
+        NeuronIn in;
+        in.V = nv.V[i];
+        in.iou = nv.iou[i];
+        in.tlast = nv.tlast[i];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) in.J[c] = GATHER ? decay_add(Jc[c], pp.decay[c], fix_to_float(acc[c])) : Jc[c];
+        float z, u = 1.f;
+        draw_noise1(nv, i, ps.n, ps.inj_base, (ps.flags & kFlagInjected) != 0, ps.prop_mode != PROP_THRESHOLD, z, u, err);
+        const NeuronOut o = lif_update(pp, in, ps.t, z, (ps.flags & kFlagUseOU) != 0);
+        nv.V[i] = o.V;
+        nv.iou[i] = o.iou;
+        nv.tlast[i] = o.tlast;
+        if constexpr (GATHER) nv.J[i] = make_float4(in.J[0], in.J[1], in.J[2], in.J[3]);
+        active = o.active;
+        vnew = o.V;
+        sp = propagated(ps.prop_mode, o.active, u, pp.noise_rate);
+    }
+    const uint32_t wprop = __ballot_sync(0xffffffffu, sp);
+    const uint32_t wact = __ballot_sync(0xffffffffu, active);
+    if ((ps.flags & kFlagSample) && nv.n_samples && valid && ps.row >= 0 && ps.row < static_cast<long long>(nv.hist_cap)) {
+        const uint32_t sbw = __ldg(nv.sample_bits + (i >> 5));
+        if ((sbw >> (i & 31u)) & 1u) {
+            const uint32_t slot = __ldg(nv.sample_pre + (i >> 5)) + __popc(sbw & ((1u << (i & 31u)) - 1u));
+            const size_t o = static_cast<size_t>(ps.row) * nv.n_samples + slot;
+            nv.hist_sspk[o] = active ? 1 : 0;
+            nv.hist_sv[o] = vnew;
+            nv.hist_siou[o] = nv.iou[i];
+        }
+    }
+    if (lane == 0) {
+        uint32_t* bits = (ps.n & 1ull) ? nv.bits1 : nv.bits0;
+        bits[base >> 5] = wprop;
+        if (ps.record) nv.rec_bits[static_cast<size_t>(ps.row) * nv.n_words + (base >> 5)] = wact;
+    }
+    if (wprop) {
+        const unsigned long long ev = warp_sum_ull(sp ? static_cast<unsigned long long>(__ldg(nv.out_deg + i)) : 0ull);
+        if (lane == 0 && ev) atomicAdd(s_events, ev);
+    }
+    if (ps.stats) {
+        const bool inc = valid && !excluded(nv, i);
+        const uint32_t pl = __shfl_sync(0xffffffffu, p, 0);
+        const bool wuni = __all_sync(0xffffffffu, !valid || (inc && p == pl)) && __any_sync(0xffffffffu, valid);
+        const int c = inc && active ? 1 : 0;
+        const long long v = inc ? v_fix(vnew) : 0;
+        if (wuni) {
+            const int cs = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(c));
+            const long long vs = warp_sum_ll(v);
+            if (lane == 0) stat_add(nv, sa, ps.row, pl, cs, vs);
+        } else if (inc) {
+            stat_add(nv, sa, ps.row, p, c, v);
+        }
+    }
+}
+
+// End of a pull CTA: its statistics and events.
+__device__ __forceinline__ void pull_flush(const NetView& nv, const PullStep& ps, const StatAcc& sa, unsigned long long* s_events) {
+    __syncthreads();
+    if (threadIdx.x == 0 && *s_events) atomicAdd(nv.events, *s_events);
+    if (ps.stats && threadIdx.x < kStatSlots) {
+        const int c = sa.cnt[threadIdx.x];
+        const long long v = sa.vs[threadIdx.x];
+        if (c || v) {
+            const size_t o = static_cast<size_t>(ps.row) * nv.n_pops + (sa.p0 + threadIdx.x);
+            if (c) atomicAdd(nv.hist_cnt + o, c);
+            atomicAdd(reinterpret_cast<unsigned long long*>(nv.hist_vsum + o), static_cast<unsigned long long>(v));
         }
     }
 }
@@ -1467,104 +1583,57 @@ lif_pull_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ t
     load_netview(s_nv, nets + s_net);
     __syncthreads();
     const NetView& nv = s_nv;
-    const float t_prev = nv.clock->t;
-    const unsigned long long n_prev = nv.clock->n;
-    const unsigned long long run_base = nv.clock->run_base;
-    const unsigned long long inj_base = nv.clock->inj_base;
-    const unsigned long long n = n_prev + 1;
-    const float t = __fadd_rn(t_prev, nv.dt);
-    const uint32_t parity = static_cast<uint32_t>(n & 1ull);
-    const uint32_t tile_first = s_tile * kPullTile;
-    const uint32_t base = tile_first + warp * 32;
-    const uint32_t i = base + lane;
     uint32_t err = 0;
-    const long long row = static_cast<long long>(n - run_base - 1);
-    bool stats = (flags & kFlagStats) != 0;
-    bool record = (flags & kFlagRecord) != 0 && nv.rec_bits != nullptr;
-    if ((stats || record) && (row < 0 || row >= static_cast<long long>(nv.hist_cap))) {
-        stats = false; record = false; err |= kErrHistOverflow;
-    }
+    const PullStep ps = pull_step(nv, flags, prop_mode, err);
+    const uint32_t tile_first = s_tile * kPullTile;
     if (tid == 0) s_p0 = find_pop(nv.pop_off, nv.n_pops, min(tile_first, nv.n - 1));
     __syncthreads();
-    StatAcc sa{s_cnt, s_vs, s_p0};
+    const StatAcc sa{s_cnt, s_vs, s_p0};
+    pull_step32<GATHER, WT, 4>(nv, ps, tile_first + warp * 32, (ps.n & 1ull) ? nv.bits0 : nv.bits1, lane, sa, &s_events, err);
+    pull_flush(nv, ps, sa, &s_events);
+    advance_clock(nv, nv.n_pad / kPullTile, ps.t, ps.n, err);
+}
 
-    long long acc[4] = {0, 0, 0, 0};
-    if constexpr (GATHER) {
-        const uint32_t* prev = parity ? nv.bits0 : nv.bits1;
-        gather32<WT>(nv, base, prev, lane, acc);
-    }
-    const bool valid = i < nv.n;
-    bool active = false, sp = false;
-    float vnew = 0.f;
-    uint32_t p = 0;
-    if (valid) {
-        p = find_pop(nv.pop_off, nv.n_pops, i);
-        PopParams pp;
-        load_pop_params(nv, p, i, pp);
-        float4 Jv = nv.J[i];
-        float* Jc = reinterpret_cast<float*>(&Jv);
-        NeuronIn in;
-        in.V = nv.V[i];
-        in.iou = nv.iou[i];
-        in.tlast = nv.tlast[i];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) in.J[c] = GATHER ? decay_add(Jc[c], pp.decay[c], fix_to_float(acc[c])) : Jc[c];
-        float z, u = 1.f;
-        draw_noise1(nv, i, n, inj_base, (flags & kFlagInjected) != 0, prop_mode != PROP_THRESHOLD, z, u, err);
-        const NeuronOut o = lif_update(pp, in, t, z, (flags & kFlagUseOU) != 0);
-        nv.V[i] = o.V;
-        nv.iou[i] = o.iou;
-        nv.tlast[i] = o.tlast;
-        if constexpr (GATHER) nv.J[i] = make_float4(in.J[0], in.J[1], in.J[2], in.J[3]);
-        active = o.active;
-        vnew = o.V;
-        sp = propagated(prop_mode, o.active, u, pp.noise_rate);
-    }
-    const uint32_t wprop = __ballot_sync(0xffffffffu, sp);
-    const uint32_t wact = __ballot_sync(0xffffffffu, active);
-    if ((flags & kFlagSample) && nv.n_samples && valid && row >= 0 && row < static_cast<long long>(nv.hist_cap)) {
-        const uint32_t sbw = __ldg(nv.sample_bits + (i >> 5));
-        if ((sbw >> (i & 31u)) & 1u) {
-            const uint32_t slot = __ldg(nv.sample_pre + (i >> 5)) + __popc(sbw & ((1u << (i & 31u)) - 1u));
-            const size_t o = static_cast<size_t>(row) * nv.n_samples + slot;
-            nv.hist_sspk[o] = active ? 1 : 0;
-            nv.hist_sv[o] = vnew;
-            nv.hist_siou[o] = nv.iou[i];
-        }
-    }
-    if (lane == 0) {
-        uint32_t* bits = parity ? nv.bits1 : nv.bits0;
-        bits[base >> 5] = wprop;
-        if (record) nv.rec_bits[static_cast<size_t>(row) * nv.n_words + (base >> 5)] = wact;
-    }
-    const unsigned long long ev = warp_sum_ull(sp ? __ldg(nv.out_deg + i) : 0u);
-    if (lane == 0 && ev) atomicAdd(&s_events, ev);
-    if (stats) {
-        const bool inc = valid && !excluded(nv, i);
-        const uint32_t pl = __shfl_sync(0xffffffffu, p, 0);
-        const bool wuni = __all_sync(0xffffffffu, !valid || (inc && p == pl)) && __any_sync(0xffffffffu, valid);
-        const int c = inc && active ? 1 : 0;
-        const long long v = inc ? v_fix(vnew) : 0;
-        if (wuni) {
-            const int cs = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(c));
-            const long long vs = warp_sum_ll(v);
-            if (lane == 0) stat_add(nv, sa, row, pl, cs, vs);
-        } else if (inc) {
-            stat_add(nv, sa, row, p, c, v);
-        }
-    }
+// The same step with the previous step's bitmap in shared memory: a network of up to
+// kPullSmemNeurons neurons fits its bitmap beside one persistent CTA per SM, so an edge costs
+// one shared-memory word instead of a dependent access to L1 or L2 -- the chain of an in-edge
+// id and its bitmap word bounded the kernel above at a quarter of the copy bandwidth.  Warps
+// take groups of 32 neurons, strided over the grid; 16 edges in flight per lane.
+constexpr int kPullSmemThreads = 768;
+constexpr uint32_t kPullSmemNeurons = 1600u * 1024u;        // 200 KiB of bitmap
+
+__device__ __forceinline__ void stage_bitmap(uint32_t* s_bits, const uint32_t* bits, uint32_t n_words) {
+    const uint4* src = reinterpret_cast<const uint4*>(bits);   // n_words is a multiple of 32
+    uint4* dst = reinterpret_cast<uint4*>(s_bits);
+    for (uint32_t q = threadIdx.x; q < n_words / 4; q += blockDim.x) dst[q] = src[q];
     __syncthreads();
-    if (tid == 0 && s_events) atomicAdd(nv.events, s_events);
-    if (stats && tid < kStatSlots) {
-        const int c = s_cnt[tid];
-        const long long v = s_vs[tid];
-        if (c || v) {
-            const size_t o = static_cast<size_t>(row) * nv.n_pops + (s_p0 + tid);
-            if (c) atomicAdd(nv.hist_cnt + o, c);
-            atomicAdd(reinterpret_cast<unsigned long long*>(nv.hist_vsum + o), static_cast<unsigned long long>(v));
-        }
-    }
-    advance_clock(nv, nv.n_pad / kPullTile, t, n, err);
+}
+
+template <int WT>
+__global__ void __launch_bounds__(kPullSmemThreads, 1)
+lif_pull_smem_kernel(const NetView* __restrict__ nets, uint32_t flags, int prop_mode) {
+    extern __shared__ __align__(16) uint32_t s_bits[];
+    __shared__ NetView s_nv;
+    __shared__ unsigned long long s_events;
+    __shared__ int s_cnt[kStatSlots];
+    __shared__ long long s_vs[kStatSlots];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_events = 0ull;
+    if (tid < kStatSlots) { s_cnt[tid] = 0; s_vs[tid] = 0; }
+    load_netview(s_nv, nets);
+    __syncthreads();
+    const NetView& nv = s_nv;
+    uint32_t err = 0;
+    const PullStep ps = pull_step(nv, flags, prop_mode, err);
+    stage_bitmap(s_bits, (ps.n & 1ull) ? nv.bits0 : nv.bits1, nv.n_words);
+    const StatAcc sa{s_cnt, s_vs, 0u};
+    const uint32_t warps = gridDim.x * (kPullSmemThreads / 32);
+    for (uint32_t g = warp * gridDim.x + blockIdx.x; g < nv.n_words; g += warps)
+        pull_step32<1, WT, 16>(nv, ps, g * 32, s_bits, lane, sa, &s_events, err);
+    pull_flush(nv, ps, sa, &s_events);
+    err = __reduce_or_sync(0xffffffffu, err);
+    if (lane == 0 && err) atomicOr(&nv.clock->err, err);
+    advance_clock(nv, gridDim.x, ps.t, ps.n, 0u);
 }
 
 // End of an exact- or fixed-push run: J <- J*decay + dJ (or dJf), the sums <- 0
@@ -1601,19 +1670,11 @@ fold_finish_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict_
     }
 }
 
-// End of a pull run: J <- J*decay + gather(last step's spikes).
-template <int WT>
-__global__ void __launch_bounds__(kPullThreads)
-gather_finish_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_prefix, uint32_t n_nets) {
-    const uint32_t k = n_nets > 1 ? find_net(tile_prefix, n_nets, blockIdx.x) : 0u;
-    const NetView& nv = nets[k];
-    const uint32_t tile = blockIdx.x - __ldg(tile_prefix + k);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t base = tile * kPullTile + warp * 32;
-    const unsigned long long n = nv.clock->n;
-    const uint32_t* last = (n & 1ull) ? nv.bits1 : nv.bits0;
+// J <- J*decay + gather(last step's spikes) for the 32 neurons from `base` on.
+template <int WT, int U>
+__device__ __forceinline__ void gather_finish32(const NetView& nv, uint32_t base, const uint32_t* last, int lane) {
     long long acc[4];
-    gather32<WT>(nv, base, last, lane, acc);
+    gather32<WT, U>(nv, base, last, lane, acc);
     const uint32_t i = base + lane;
     if (i < nv.n) {
         const uint32_t p = find_pop(nv.pop_off, nv.n_pops, i);
@@ -1625,6 +1686,29 @@ gather_finish_kernel(const NetView* __restrict__ nets, const uint32_t* __restric
         for (int c = 0; c < 4; ++c) Jc[c] = decay_add(Jc[c], pp.decay[c], fix_to_float(acc[c]));
         nv.J[i] = Jv;
     }
+}
+
+// End of a pull run.
+template <int WT>
+__global__ void __launch_bounds__(kPullThreads)
+gather_finish_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_prefix, uint32_t n_nets) {
+    const uint32_t k = n_nets > 1 ? find_net(tile_prefix, n_nets, blockIdx.x) : 0u;
+    const NetView& nv = nets[k];
+    const uint32_t tile = blockIdx.x - __ldg(tile_prefix + k);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t* last = (nv.clock->n & 1ull) ? nv.bits1 : nv.bits0;
+    gather_finish32<WT, 4>(nv, tile * kPullTile + warp * 32, last, lane);
+}
+
+template <int WT>
+__global__ void __launch_bounds__(kPullSmemThreads, 1)
+gather_finish_smem_kernel(const NetView* __restrict__ nets) {
+    extern __shared__ __align__(16) uint32_t s_bits[];
+    const NetView& nv = nets[0];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    stage_bitmap(s_bits, (nv.clock->n & 1ull) ? nv.bits1 : nv.bits0, nv.n_words);
+    for (uint32_t g = warp * gridDim.x + blockIdx.x; g < nv.n_words; g += gridDim.x * (kPullSmemThreads / 32))
+        gather_finish32<WT, 16>(nv, g * 32, s_bits, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -1922,8 +2006,41 @@ static void pull_dispatch(const LaunchBatch& b, int wt, uint32_t flags, int prop
     }
 }
 
+// Whether a launch's bitmap goes to shared memory, and the bytes it takes (0: it stays in L2).
+static uint32_t pull_smem_bytes(const LaunchBatch& b) {
+    const uint32_t neurons = b.pull_tiles_total * kPullTile;
+    if (b.n_nets != 1 || neurons > kPullSmemNeurons) return 0;
+    return (neurons + kPad - 1) / kPad * kPad / 8;
+}
+
+template <class F>
+static cudaError_t pull_smem_attr(F fn, uint32_t bytes) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
+template <int WT>
+static cudaError_t pull_smem_launch(const LaunchBatch& b, uint32_t bytes, bool finish, uint32_t flags, int prop_mode, cudaStream_t s) {
+    cudaError_t e = finish ? pull_smem_attr(gather_finish_smem_kernel<WT>, bytes) : pull_smem_attr(lif_pull_smem_kernel<WT>, bytes);
+    if (e != cudaSuccess) return e;
+    if (finish) gather_finish_smem_kernel<WT><<<b.sm_count, kPullSmemThreads, bytes, s>>>(b.nets);
+    else lif_pull_smem_kernel<WT><<<b.sm_count, kPullSmemThreads, bytes, s>>>(b.nets, flags, prop_mode);
+    return cudaGetLastError();
+}
+
+static cudaError_t pull_smem_dispatch(const LaunchBatch& b, int wt, uint32_t bytes, bool finish, uint32_t flags, int prop_mode,
+                                      cudaStream_t s) {
+    switch (wt) {
+        case W_F32: return pull_smem_launch<W_F32>(b, bytes, finish, flags, prop_mode, s);
+        case W_BF16: return pull_smem_launch<W_BF16>(b, bytes, finish, flags, prop_mode, s);
+        case W_F16: return pull_smem_launch<W_F16>(b, bytes, finish, flags, prop_mode, s);
+        default: return pull_smem_launch<W_U8>(b, bytes, finish, flags, prop_mode, s);
+    }
+}
+
 cudaError_t launch_pull(const LaunchBatch& b, int gather, int wt, uint32_t flags, int prop_mode, cudaStream_t s) {
     if (b.pull_tiles_total == 0) return cudaSuccess;
+    const uint32_t bytes = pull_smem_bytes(b);
+    if (gather && bytes) return pull_smem_dispatch(b, wt, bytes, false, flags, prop_mode, s);
     if (gather) pull_dispatch<1>(b, wt, flags, prop_mode, s); else pull_dispatch<0>(b, wt, flags, prop_mode, s);
     return cudaGetLastError();
 }
@@ -1948,6 +2065,7 @@ cudaError_t launch_fold_finish(const LaunchBatch& b, int acc, cudaStream_t s) {
 
 cudaError_t launch_gather_finish(const LaunchBatch& b, int wt, cudaStream_t s) {
     if (b.pull_tiles_total == 0) return cudaSuccess;
+    if (const uint32_t bytes = pull_smem_bytes(b)) return pull_smem_dispatch(b, wt, bytes, true, 0u, 0, s);
     const dim3 grid(b.pull_tiles_total), block(kPullThreads);
     switch (wt) {
         case W_F32: gather_finish_kernel<W_F32><<<grid, block, 0, s>>>(b.nets, b.pull_prefix, b.n_nets); break;
