@@ -1009,13 +1009,8 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
                     DTB_TRY(timed_launch(2, [&] { return launch_pull(b, first ? 0 : 1, wt, kflags, pm, stream); }));
                     continue;
                 }
-                for (uint32_t k = 0; k < ts; ++k) {
-                    // substeps after the first fold nothing new: J decays with no input
-                    const int jm = jmode_of(rq.syn_mode, first && k == 0);
-                    const int jmk = k == 0 ? jm : (jm == J_ASIS ? jmode_of(rq.syn_mode, false) : jm);
-                    const uint32_t f = ts > 1 ? (kflags | substep_flags(k, ts)) : kflags;
-                    DTB_TRY(timed_launch(0, [&] { return launch_lif(b, jmk, f, pm, stream); }));
-                }
+                const uint32_t f = ts > 1 ? (kflags | substep_flags(ts)) : kflags;
+                DTB_TRY(timed_launch(0, [&] { return launch_lif(b, jmode_of(rq.syn_mode, first), f, pm, stream); }));
                 if (tuning && tune_at == done + s) {
                     DTB_TRY(tune_push(b, acc));
                     if (!push_tuned[acc]) tune_at = tune_acc[acc].next_step(tune_at);
@@ -1041,7 +1036,7 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
             DTB_CU(cudaGraphLaunch(graph, stream));
             ++graph_launches;
             // launches of the replayed chunk, counted as the eager path does
-            chunk_launches = rows * (ts + 1u + (isyn_any ? 1u : 0u)) +
+            chunk_launches = rows * (2u + (isyn_any ? 1u : 0u)) +
                              (last_chunk && acc != ACC_FLOAT ? 1u : 0u);
         } else if (graphable && std::memcmp(key, seen_key, sizeof(key)) == 0 && ++seen_count >= 2 &&
                    seen_ms_per_step < kGraphMaxMsPerStep) {

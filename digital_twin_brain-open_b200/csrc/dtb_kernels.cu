@@ -333,7 +333,10 @@ __device__ __forceinline__ uint32_t lif_next_tile(uint32_t gt, uint32_t chunk, u
 __device__ __forceinline__ void local_prep(const NetView* __restrict__ nets, const LocalPlan& lp, uint32_t n_nets, uint32_t count,
                                            uint32_t* s_warp);
 
-template <int JM>
+// SUBS: all substeps of a step (RunRequest.t_steps > 1) on a tile while it is in shared memory --
+// no neuron depends on another between them, so one launch takes the step's substeps with one
+// pass over the state instead of one launch and pass each.
+template <int JM, bool SUBS>
 __global__ void __launch_bounds__(kLifThreads, kLifCtasPerSm)
 lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_prefix,
            const uint32_t* __restrict__ vbase, uint32_t n_nets, uint32_t total_tiles, SpikeList sl, uint32_t flags,
@@ -350,12 +353,10 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     const bool use_ou = (flags & kFlagUseOU) != 0;
     const bool need_u = prop_mode != PROP_THRESHOLD;
     const bool injected = (flags & kFlagInjected) != 0;
-    // substep k of ts: spikes OR into the step's bitmap and list (a neuron enters the list
-    // once), counts are of neurons newly spiking, V statistics and samples come from the
-    // last substep, and the clock's step count advances after it (dist_simulator.cpp:2085-2112)
-    const uint32_t sub = (flags >> kSubShift) & 0xFFu;
-    const uint32_t ts = max(1u, (flags >> kTsShift) & 0xFFu);
-    const bool last_sub = sub + 1 >= ts;
+    // substeps: spikes OR into the step's bitmap and list (a neuron enters the list once),
+    // counts are of neurons newly spiking, V statistics and samples come from the last
+    // substep, and the clock's step count advances once (dist_simulator.cpp:2085-2112)
+    const uint32_t ts = SUBS ? max(1u, (flags >> kTsShift) & 0xFFu) : 1u;
     uint32_t late = 0;                 // a bulk-copy wait ran out
     uint32_t done_here = 0;            // tiles of cur_net this CTA finished (thread 0's ticket)
     float t_last_tile = 0.f;
@@ -422,7 +423,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         const unsigned long long inj_base = nv.clock->inj_base;
         const uint32_t p_tile = __ldg(nv.tile_pop + tile);
         const unsigned long long n = n_prev + 1;
-        const float t = __fadd_rn(t_prev, nv.dt);
+        float t = __fadd_rn(t_prev, nv.dt);
         const uint32_t parity = static_cast<uint32_t>(n & 1ull);
         uint32_t err = 0;
         const long long row = static_cast<long long>(n - run_base - 1);
@@ -431,19 +432,10 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         if ((stats || record) && (row < 0 || row >= static_cast<long long>(nv.hist_cap))) {
             stats = false; record = false; err |= kErrHistOverflow;
         }
-        const bool sample = (flags & kFlagSample) && nv.n_samples && row >= 0 && row < static_cast<long long>(nv.hist_cap) &&
-                            last_sub;
+        const bool sample = (flags & kFlagSample) && nv.n_samples && row >= 0 && row < static_cast<long long>(nv.hist_cap);
         StatAcc sa{s_cnt[it & 1u], s_vs[it & 1u], p_tile};
         float z[4], u[4] = {1.f, 1.f, 1.f, 1.f};
-        draw_noise(nv, tile_first, tid, n, inj_base, injected, need_u, z, u, err, sub, ts);
-        // propagated spikes of this step's earlier substeps, one word per k of this warp
-        uint32_t old_w[4] = {0u, 0u, 0u, 0u};
-        if (sub) {
-            const uint32_t* bits = parity ? nv.bits1 : nv.bits0;
-            const uint32_t word0 = (tile_first >> 5) + (tid >> 5);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) old_w[k] = bits[word0 + (kSlotsPerTile / 32) * k];
-        }
+        draw_noise(nv, tile_first, tid, n, inj_base, injected, need_u, z, u, err, 0u, ts);
         const uint32_t phase = (it / kLifStages) & 1u;
         if (!mbar_wait_bounded(&s_bar[stg], phase)) {
             late = 1;
@@ -458,8 +450,9 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         float* sT = st + 2 * kLifTile + tid;
         float4* sJ = reinterpret_cast<float4*>(st + 3 * kLifTile) + tid;
 
-        uint32_t nib_prop = 0, nib_act = 0;
         uint32_t ev = 0;                   // out-degrees of this thread's (at most four) spiking neurons
+        // spikes of the step's earlier substeps, propagated and threshold, one word per k of this warp
+        uint32_t old_w[4] = {0u, 0u, 0u, 0u}, old_act[4] = {0u, 0u, 0u, 0u};
         uint32_t p = p_tile;
         const uint32_t i_first = min(i0, nv.n - 1);
         while (p + 1 < nv.n_pops && __ldg(nv.pop_off + p + 1) <= i_first) ++p;
@@ -468,6 +461,15 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         int cnt_acc = 0, cnt_nxt = 0;          // neurons of p_first, and of p_first + 1
         long long vs_acc = 0, vs_nxt = 0;
         PopParams pp;
+        uint32_t wtotal = 0;               // neurons of the warp new to the step's list
+        for (uint32_t sub = 0; sub < ts; ++sub) {
+        const bool last_sub = !SUBS || sub + 1 == ts;
+        if (SUBS && sub) {
+            t = __fadd_rn(t, nv.dt);
+            draw_noise(nv, tile_first, tid, n, inj_base, injected, need_u, z, u, err, sub, ts);
+            p = p_first;
+        }
+        uint32_t nib_prop = 0, nib_act = 0;
         load_pop_params(nv, p, i_first, pp);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -485,7 +487,13 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
             in.V = sV[ks];
             in.iou = sI[ks];
             in.tlast = sT[ks];
-            if constexpr (JM == J_FOLD) {
+            if (SUBS && sub && JM != J_DIRECT) {
+                // nothing arrives between substeps: J decays
+                in.J[0] = decay_add(Jk.x, pp.decay[0], 0.0f);
+                in.J[1] = decay_add(Jk.y, pp.decay[1], 0.0f);
+                in.J[2] = decay_add(Jk.z, pp.decay[2], 0.0f);
+                in.J[3] = decay_add(Jk.w, pp.decay[3], 0.0f);
+            } else if constexpr (JM == J_FOLD) {
                 longlong2* dq = reinterpret_cast<longlong2*>(nv.dJ + static_cast<size_t>(i) * 4);
                 const longlong2 d01 = dq[0], d23 = dq[1];
                 in.J[0] = decay_add(Jk.x, pp.decay[0], fix_to_float(d01.x));
@@ -512,7 +520,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
             if constexpr (JM == J_DIRECT) {
                 sJ[ks] = make_float4(__fmul_rn(in.J[0], pp.decay[0]), __fmul_rn(in.J[1], pp.decay[1]),
                                      __fmul_rn(in.J[2], pp.decay[2]), __fmul_rn(in.J[3], pp.decay[3]));
-            } else if constexpr (JM == J_FOLD || JM == J_FIXF) {
+            } else if constexpr (JM == J_FOLD || JM == J_FIXF || SUBS) {
                 sJ[ks] = make_float4(in.J[0], in.J[1], in.J[2], in.J[3]);
             }
             const bool sp = propagated(prop_mode, o.active, u[k], pp.noise_rate);
@@ -521,7 +529,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
             nib_act |= static_cast<uint32_t>(o.active) << k;
             if (sp && !seen) ev += __ldg(nv.out_deg + i);
             // sampled neurons (stat_samples_kernel, src/stage/stat_result.cpp:393-431)
-            if (sample) {
+            if (sample && last_sub) {
                 const uint32_t sbw = __ldg(nv.sample_bits + (i >> 5)), sh = i & 31u;
                 if ((sbw >> sh) & 1u) {
                     const size_t so = static_cast<size_t>(row) * nv.n_samples + __ldg(nv.sample_pre + (i >> 5)) +
@@ -550,24 +558,25 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         // ---- spike bitmaps and list: step k of a warp covers one 32-neuron word
         //      (propagated: parity buffer and one slot range per warp in the list;
         //      threshold: history row)
-        uint32_t wtotal = 0;               // neurons of the warp new to the step's list
         {
             uint32_t* bits = parity ? nv.bits1 : nv.bits0;
             const uint32_t word0 = (tile_first >> 5) + (tid >> 5);
             uint32_t wprop[4];
+            wtotal = 0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint32_t all = __ballot_sync(0xffffffffu, (nib_prop >> k) & 1u);
                 wprop[k] = all & ~old_w[k];                     // new to the step's list
                 wtotal += __popc(wprop[k]);
                 const uint32_t wact = __ballot_sync(0xffffffffu, (nib_act >> k) & 1u);
-                if (lane == 0) {
+                if (lane == 0 && last_sub) {
                     const uint32_t word = word0 + (kSlotsPerTile / 32) * k;
                     bits[word] = all | old_w[k];
-                    if (record) {
-                        uint32_t* rw = nv.rec_bits + static_cast<size_t>(row) * nv.n_words + word;
-                        *rw = sub ? (*rw | wact) : wact;
-                    }
+                    if (record) nv.rec_bits[static_cast<size_t>(row) * nv.n_words + word] = wact | old_act[k];
+                }
+                if constexpr (SUBS) {
+                    old_w[k] |= all;
+                    old_act[k] |= wact;
                 }
             }
             if ((flags & kFlagList) && wtotal) {
@@ -599,6 +608,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
                 }
             }
         }
+        }
         // ---- population statistics: one sum per warp when the warp's neurons share a
         //      population, else one per (warp, population) by a segmented reduction
         if (stats) {
@@ -613,7 +623,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
                 warp_stat_segments(nv, sa, row, p_first + 1, cnt_nxt != 0 || vs_nxt != 0, cnt_nxt, vs_nxt, lane);
             }
         }
-        const unsigned long long wev = wtotal ? warp_sum_ull(ev) : 0ull;
+        const unsigned long long wev = SUBS || wtotal ? warp_sum_ull(ev) : 0ull;
         if (lane == 0 && wev) atomicAdd(nv.events, wev);
 
         // barrier B: the stage holds the finished tile; store it, flush statistics
@@ -623,7 +633,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
             bulk_store(nv.V + tile_first, st, kLifTile * sizeof(float));
             bulk_store(nv.iou + tile_first, st + kLifTile, kLifTile * sizeof(float));
             bulk_store(nv.tlast + tile_first, st + 2 * kLifTile, kLifTile * sizeof(float));
-            if constexpr (JM != J_ASIS) bulk_store(nv.J + tile_first, st + 3 * kLifTile, kLifTile * sizeof(float4));
+            if constexpr (JM != J_ASIS || SUBS) bulk_store(nv.J + tile_first, st + 3 * kLifTile, kLifTile * sizeof(float4));
             bulk_commit();
         }
         if (stats && tid < kStatSlots) {
@@ -641,7 +651,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
         if (lane == 0 && err) atomicOr(&nv.clock->err, err);
         if (tid == 0) {
             t_last_tile = t;
-            n_last_tile = last_sub ? n : n_prev;
+            n_last_tile = n;
             ++done_here;
         }
     }
@@ -653,7 +663,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     }
     // the CTA that finishes the launch's last network hands the step's list to the push kernel,
     // empties it for the next step, and prepares the windows' work units
-    if ((flags & kFlagList) && last_sub) {
+    if (flags & kFlagList) {
         __shared__ uint32_t s_warp[33];
         __shared__ uint32_t s_published;               // list length + 1 in the last CTA, else 0
         if (tid == 0) {
@@ -1830,7 +1840,8 @@ cudaError_t launch_lif(const LaunchBatch& b, int jmode, uint32_t flags, int prop
     if (e != cudaSuccess) return e;
     const uint32_t bit = 1u << (dev & 31);
     if (!(attr_set.load() & bit)) {
-        for (auto fn : {lif_kernel<J_DIRECT>, lif_kernel<J_FOLD>, lif_kernel<J_ASIS>, lif_kernel<J_FIXF>}) {
+        for (auto fn : {lif_kernel<J_DIRECT, false>, lif_kernel<J_FOLD, false>, lif_kernel<J_ASIS, false>, lif_kernel<J_FIXF, false>,
+                        lif_kernel<J_DIRECT, true>, lif_kernel<J_FOLD, true>, lif_kernel<J_ASIS, true>, lif_kernel<J_FIXF, true>}) {
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLifSmem));
             if (e != cudaSuccess) return e;
         }
@@ -1839,11 +1850,15 @@ cudaError_t launch_lif(const LaunchBatch& b, int jmode, uint32_t flags, int prop
     const uint32_t T = b.lif_tiles_total;
     const uint32_t chunk = std::max(1u, b.lif_chunk);
     const dim3 grid(std::min((T + chunk - 1) / chunk, b.lif_ctas)), block(kLifThreads);
+    auto go = [&](auto fn) {
+        fn<<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local);
+    };
+    const bool subs = ((flags >> kTsShift) & 0xFFu) > 1u;
     switch (jmode) {
-        case J_DIRECT: lif_kernel<J_DIRECT><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
-        case J_FOLD: lif_kernel<J_FOLD><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
-        case J_FIXF: lif_kernel<J_FIXF><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
-        default: lif_kernel<J_ASIS><<<grid, block, kLifSmem, s>>>(b.nets, b.lif_prefix, b.vbase, b.n_nets, T, b.spikes, flags, prop_mode, b.tile_net, chunk, b.local); break;
+        case J_DIRECT: subs ? go(lif_kernel<J_DIRECT, true>) : go(lif_kernel<J_DIRECT, false>); break;
+        case J_FOLD: subs ? go(lif_kernel<J_FOLD, true>) : go(lif_kernel<J_FOLD, false>); break;
+        case J_FIXF: subs ? go(lif_kernel<J_FIXF, true>) : go(lif_kernel<J_FIXF, false>); break;
+        default: subs ? go(lif_kernel<J_ASIS, true>) : go(lif_kernel<J_ASIS, false>); break;
     }
     return cudaGetLastError();
 }
