@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(kDaThreads)
 da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, uint32_t vb, uint32_t width, const float* __restrict__ w,
                 const float* __restrict__ y, const float* __restrict__ noise, double sigma, double* __restrict__ mean,
                 double* __restrict__ temp, double* __restrict__ innov, double* __restrict__ colsum) {
-    __shared__ double s_part[kDaThreads];
+    __shared__ double s_part[kDaThreads], s_mean[kDaThreads];
     const uint32_t groups = kDaThreads / width, g = threadIdx.x / width, x = threadIdx.x % width;
     const uint32_t v0 = blockIdx.x * vb, nv = min(vb, V - v0), cols = nv * S;
     const size_t row = static_cast<size_t>(V) * S;
@@ -56,12 +56,19 @@ da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, uint32_t vb, uint32_t width,
         const double m = meet(acc) / E;
         // the voxel's last column: its mean and variance
         const float* last = w + static_cast<size_t>(v) * S + S - 1;
-        double al = 0.0;
-        if (in) {
+        double ml;
+        if (cols <= width) {                                 // it is another lane's column of this pass
+            if (in && g == 0) s_mean[x] = m;
+            __syncthreads();
+            ml = s_mean[in ? vl * S + S - 1 : 0u];
+        } else {
+            double al = 0.0;
+            if (in) {
 #pragma unroll 4
-            for (uint32_t e = g; e < E; e += groups) al += last[e * row];
+                for (uint32_t e = g; e < E; e += groups) al += last[e * row];
+            }
+            ml = meet(al) / E;
         }
-        const double ml = meet(al) / E;
         double cx = 0.0;
         if (in) {
 #pragma unroll 4
@@ -74,6 +81,7 @@ da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, uint32_t vb, uint32_t width,
         double cs = 0.0;
         if (in) {
             const bool lead = col % S == S - 1;              // the lane that writes the voxel's temp and innov
+#pragma unroll 4
             for (uint32_t e = g; e < E; e += groups) {
                 const double l = last[e * row];
                 const double t = (l - ml) / cxx / (E - 1);
@@ -92,10 +100,10 @@ da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, uint32_t vb, uint32_t width,
     }
 }
 
-// G[e][f] = sum_v I[e,v] T[f,v] / V.  A CTA makes an 8 x 8 tile: rows of 64 voxels of both
+// G[e][f] = sum_v I[e,v] T[f,v] / V.  A CTA makes an 8 x 8 tile: rows of 256 voxels of both
 // factors are staged in shared memory and four threads share a product's voxels (a warp per
 // product re-read both rows for each of the E^2 products).
-constexpr int kGainTile = 8, kGainVox = 64;
+constexpr int kGainTile = 8, kGainVox = 256;
 __global__ void __launch_bounds__(kDaThreads)
 da_gain_kernel(uint32_t E, uint32_t V, const double* __restrict__ innov, const double* __restrict__ temp,
                double* __restrict__ gain) {
