@@ -128,6 +128,7 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
     uint64_t edges = 0;
     for (const Engine* e : m) edges += e->n_edges;
     dense_min = dense_min_spikes(edges, total);
+    edges_total = edges;
     windows_total = windows;
     lb.local = LocalPlan{d_prefix + 3 * (n + 1), windows, dense_min, 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch};
     lb.sm_count = static_cast<uint32_t>(sm_count);
@@ -219,7 +220,7 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
         lb.local.dense_min = window_always ? 1u : dense_min;
         lb.local.always = window_always ? 1u : 0u;
         DTB_CU(push_prepare(acc, wt, push_cfg, sm_count, &push_ctas));
-        if (autotune && !push_tuned[acc]) {
+        if (autotune && !push_tuned[acc] && worth_tuning(edges_total)) {
             const uint64_t settle = 300;
             const uint64_t st = m[0]->steps;
             tune_at = st >= settle ? 1 : (settle - st < rq.iters ? settle - st : ~0ull);

@@ -966,7 +966,7 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
     uint64_t tune_at = ~0ull;   // run-relative step at which the push variants are timed
     if (!pull) {
         DTB_CU(push_prepare(acc, wt, push_cfg, sm_count, &push_ctas));
-        if (autotune && !push_tuned[acc] && ts == 1) {
+        if (autotune && !push_tuned[acc] && ts == 1 && worth_tuning(n_edges)) {
             // time the variants on a live spike list, once the network has left its quiet start
             const uint64_t settle = 300;
             tune_at = steps >= settle ? 1 : (settle - steps < rq.iters ? settle - steps : ~0ull);
