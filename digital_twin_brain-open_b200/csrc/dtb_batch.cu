@@ -10,7 +10,7 @@
 // nothing extra: tiles and spiking rows are distributed over the whole GPU.
 //
 // A window of steps of a push mode is captured once into a CUDA graph (2 kernel
-// nodes per step, 5 with the population-local push) and replayed per window; the
+// nodes per step) and replayed per window; the
 // push variant is chosen by the same on-line autotuner as a single engine's, on
 // the batch's own spike list.
 #include <algorithm>

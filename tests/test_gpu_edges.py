@@ -77,3 +77,12 @@ def test_pull_equals_exact_push(gpu, n, pops, degree):
     assert res[0][0].sum() + res[0][2].sum() >= n // 2        # most neurons fire at least once
     for x, y in zip(*res):
         assert (x is None and y is None) or np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("ts", [1, 4, 255])
+def test_kernel_times_with_substeps(gpu, ts):
+    """Per-kernel timing of a run with substeps and synaptic-current outputs: every launch of a step
+    has its pair of events."""
+    with E.Engine.structured(nw.structured_spec(3000, 3, 50, seed=1)) as eng:
+        r = eng.run(7, t_steps=ts, imean=True, time_kernels=True, syn_mode=E.SYN_PUSH_FIXED)
+        assert all(k > 0 for k in (r.kernel_ms[0], r.kernel_ms[1], r.kernel_ms[3])) and r.imeans.shape == (7, 3)
