@@ -591,9 +591,11 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
                     base += __popc(wprop[k]);
                 }
                 // spiking rows per population, for the windows: one reduction per warp, or per
-                // neuron in the few warps that hold a population boundary
+                // neuron in the few warps that hold a population boundary.  The last population
+                // is the warp's largest p, not lane 31's: in the network's last words lane 31 can
+                // be past the end while lower lanes step a later population.
                 if (lp.windows) {
-                    const uint32_t pa = __shfl_sync(0xffffffffu, p_first, 0), pb = __shfl_sync(0xffffffffu, p, 31);
+                    const uint32_t pa = __shfl_sync(0xffffffffu, p_first, 0), pb = __reduce_max_sync(0xffffffffu, p);
                     if (pa == pb) {
                         if (lane == 0) atomicAdd(nv.pop_live + pa, wtotal);
                     } else {
@@ -1048,7 +1050,7 @@ __device__ __forceinline__ void push_windows(const NetView* __restrict__ nets, c
         }
         const uint32_t unit_rows = unit_rows_of(unit, W.least, FIX ? 2u : 1u);
         const uint32_t r_lo = (u - upre[gw]) * unit_rows;
-        const uint32_t r_hi = min(r_lo + unit_rows, rows_of[gw]);
+        uint32_t r_hi = min(r_lo + unit_rows, rows_of[gw]);
         // rows with population rank in [r_lo, r_hi): prefix over the population's bitmap
         const uint32_t* bits = (W.nv->clock->n & 1ull) ? W.nv->bits1 : W.nv->bits0;
         const uint32_t w_lo = W.p_lo >> 5, w_hi = (W.p_hi + 31) >> 5;
@@ -1058,6 +1060,7 @@ __device__ __forceinline__ void push_windows(const NetView* __restrict__ nets, c
         for (uint32_t wi = my_lo; wi < my_hi; ++wi) c += __popc(pop_word(bits, wi, W.p_lo, W.p_hi));
         uint32_t total;
         uint32_t rank = group_exclusive_scan(c, s_warp, &total, nt);
+        r_hi = min(r_hi, total);           // never past the rows the bitmap holds
         for (uint32_t wi = my_lo; wi < my_hi && rank < r_hi; ++wi) {
             uint32_t m = pop_word(bits, wi, W.p_lo, W.p_hi);
             if (rank + __popc(m) <= r_lo) { rank += __popc(m); continue; }
@@ -1069,7 +1072,7 @@ __device__ __forceinline__ void push_windows(const NetView* __restrict__ nets, c
             }
         }
         group_sync(nt);
-        const uint32_t nrows = r_hi - r_lo;
+        const uint32_t nrows = r_hi > r_lo ? r_hi - r_lo : 0u;
         // span of every row of the unit: [out_ptr[j] + woff[k], out_ptr[j] + woff[k + 1])
         const NetView& nv = *W.nv;
         for (uint32_t r = threadIdx.x; r < nrows; r += nt) {

@@ -36,6 +36,33 @@ def test_tuned_window_form_gives_the_register_pushs_bits(gpu, n, pops, degree, w
         assert np.array_equal(v0, v) and np.array_equal(j0, j)
 
 
+@pytest.mark.parametrize("sizes", [(2306, 8), (2306, 6, 2), (4864, 33, 1), (1025, 1281, 9)])
+def test_windows_with_a_small_last_population(gpu, sizes):
+    """Populations that end inside a warp's 32-neuron word at the end of the network: the rows a
+    population hands to its windows are the rows it has.  The windows of every step, with the
+    fixed-point push, must leave the register push's bits; every population has windows (own-population
+    spans of 36 synapses and more a neuron) and every neuron fires, so a miscounted row shows."""
+    rng = np.random.default_rng(sum(sizes))
+    n, off = sum(sizes), np.concatenate([[0], np.cumsum(sizes)])
+    pop = np.repeat(np.arange(len(sizes)), sizes)
+    own, rest = 36, 8
+    post = np.repeat(np.arange(n, dtype=np.uint32), own + rest)
+    lo, width = off[pop][:, None], np.asarray(sizes)[pop][:, None]
+    pre = np.concatenate([lo + rng.integers(0, 2 ** 31, (n, own)) % width, rng.integers(0, n, (n, rest))], 1)
+    net = dict(property=nw.lif_property(n, pop), input_neuron_idx=pre.reshape(-1).astype(np.uint32), output_neuron_idx=post,
+               input_channel_offset=np.zeros(post.size, np.uint8), weight=rng.random((post.size, 2), dtype=np.float32))
+    res = []
+    for variant in ((E.PUSH_REG, 8), (E.PUSH_LOCAL, 8), (E.PUSH_LOCAL, 2016)):
+        with E.Engine.from_arrays(net, seed=5, ou=(3.0, 0.5, 10.0)) as eng:
+            assert eng.info().local_windows == len(sizes)
+            eng.set_push_variant(*variant)
+            r = eng.run(400, syn_mode=E.SYN_PUSH_FIXED)
+            res.append((r.freqs, r.events, eng.read_state(E.STATE_V), eng.read_state(E.STATE_J)))
+    assert (res[0][0].sum(0) >= np.asarray(sizes)).all()
+    for other in res[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(res[0], other))
+
+
 @pytest.mark.parametrize("out_degree", [1, 255, 256, 257, 2047, 2049, 5000])
 def test_few_long_rows_are_cut_into_parts(gpu, out_degree):
     """A step whose only spikes are three neurons of a given out-degree (a strong drive on them
