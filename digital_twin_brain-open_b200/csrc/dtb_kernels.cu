@@ -587,7 +587,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
                 const uint32_t vb = __ldg(vbase + net) + i0;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    if ((nib_prop >> k) & 1u) sl.list[base + __popc(wprop[k] & below)] = vb + kSlotsPerTile * k;
+                    if ((wprop[k] >> lane) & 1u) sl.list[base + __popc(wprop[k] & below)] = vb + kSlotsPerTile * k;
                     base += __popc(wprop[k]);
                 }
                 // spiking rows per population, for the windows: one reduction per warp, or per

@@ -55,6 +55,29 @@ def test_substeps_bit_exact(gpu, syn, ts):
         assert inf.step == steps and inf.t == o.t     # the clock advanced by dt / ts per substep
 
 
+@pytest.mark.parametrize("syn", [E.SYN_PUSH_EXACT, E.SYN_PUSH_FIXED], ids=["exact", "fixed"])
+def test_neurons_that_spike_in_several_substeps(gpu, syn):
+    """Without a refractory period a neuron over threshold spikes again in the next substep: it is
+    propagated once, from one entry of the step's list.  3072 neurons fill the LIF kernel's tiles, so
+    a list entry written twice would also pass the list's end."""
+    n, steps, ts = 3072, 60, 4
+    net = nw.make_uniform_block(n, 40, seed=6)
+    net["property"][:, 5] = 0.0                     # T_ref
+    net["property"][:, 10:14] *= 0.01               # the drive, not the recurrent input, makes them fire
+    z, _ = lo.torch_noise_stream(3, n, steps * ts, False)
+    ou = (3.0, 0.5, 5.0)
+    o = lo.LifOracle(net, dt=float(np.float32(0.1) / np.float32(ts)), ou=ou)
+    rec = np.array([o.step_substeps(z[ts * s:ts * (s + 1)]) for s in range(steps)])
+    assert rec[40:].mean() > 0.8 and (rec.sum(1) == n).any()     # they keep firing, substep after substep
+    with E.Engine.from_arrays(net, seed=1, ou=ou) as eng:
+        eng.set_noise_injected(z)
+        r = eng.run(steps, record_spikes=True, syn_mode=syn, t_steps=ts)
+        assert np.array_equal(r.spikes, rec)
+        assert r.events == int((rec * np.bincount(net["input_neuron_idx"], minlength=n)).sum())
+        assert np.array_equal(eng.read_state(E.STATE_J), o.J.T)
+        assert np.array_equal(eng.read_state(E.STATE_V), o.V)
+
+
 def test_substeps_float_push_until_divergence(gpu):
     net = nw.make_uniform_block(3000, 100, seed=2)
     steps, ts = 300, 2
