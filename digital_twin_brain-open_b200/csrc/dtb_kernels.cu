@@ -2031,15 +2031,32 @@ static uint32_t pull_smem_bytes(const LaunchBatch& b) {
     return (neurons + kPad - 1) / kPad * kPad / 8;
 }
 
-template <class F>
-static cudaError_t pull_smem_attr(F fn, uint32_t bytes) {
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+// The opt-in to the largest bitmap's shared memory, once per device for every kernel of the form:
+// the limit belongs to the function, so a size per launch would let one thread's small network
+// lower it between another's setting and launch.
+static cudaError_t pull_smem_prepare() {
+    static std::atomic<uint32_t> attr_set{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint32_t bit = 1u << (dev & 31);
+    if (attr_set.load() & bit) return cudaSuccess;
+    constexpr int most = static_cast<int>(kPullSmemNeurons / 8);
+    for (auto fn : {lif_pull_smem_kernel<W_F32>, lif_pull_smem_kernel<W_BF16>, lif_pull_smem_kernel<W_F16>, lif_pull_smem_kernel<W_U8>}) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return e;
+    }
+    for (auto fn : {gather_finish_smem_kernel<W_F32>, gather_finish_smem_kernel<W_BF16>, gather_finish_smem_kernel<W_F16>,
+                    gather_finish_smem_kernel<W_U8>}) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return e;
+    }
+    attr_set.fetch_or(bit);
+    return cudaSuccess;
 }
 
 template <int WT>
 static cudaError_t pull_smem_launch(const LaunchBatch& b, uint32_t bytes, bool finish, uint32_t flags, int prop_mode, cudaStream_t s) {
-    cudaError_t e = finish ? pull_smem_attr(gather_finish_smem_kernel<WT>, bytes) : pull_smem_attr(lif_pull_smem_kernel<WT>, bytes);
-    if (e != cudaSuccess) return e;
     if (finish) gather_finish_smem_kernel<WT><<<b.sm_count, kPullSmemThreads, bytes, s>>>(b.nets);
     else lif_pull_smem_kernel<WT><<<b.sm_count, kPullSmemThreads, bytes, s>>>(b.nets, flags, prop_mode);
     return cudaGetLastError();
@@ -2047,6 +2064,8 @@ static cudaError_t pull_smem_launch(const LaunchBatch& b, uint32_t bytes, bool f
 
 static cudaError_t pull_smem_dispatch(const LaunchBatch& b, int wt, uint32_t bytes, bool finish, uint32_t flags, int prop_mode,
                                       cudaStream_t s) {
+    const cudaError_t e = pull_smem_prepare();
+    if (e != cudaSuccess) return e;
     switch (wt) {
         case W_F32: return pull_smem_launch<W_F32>(b, bytes, finish, flags, prop_mode, s);
         case W_BF16: return pull_smem_launch<W_BF16>(b, bytes, finish, flags, prop_mode, s);

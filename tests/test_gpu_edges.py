@@ -79,6 +79,34 @@ def test_pull_equals_exact_push(gpu, n, pops, degree):
         assert (x is None and y is None) or np.array_equal(x, y)
 
 
+def test_pulls_of_two_sizes_from_two_threads(gpu):
+    """Two threads step a small network and one with the largest bitmap that shared memory takes:
+    each gives the bits it gives alone."""
+    import threading
+    specs = [nw.structured_spec(n, 3, 5, seed=n) for n in (2_000, 1_638_400)]
+
+    def steps(eng, runs):
+        out = [eng.run(3, syn_mode=E.SYN_PULL).freqs for _ in range(runs)]
+        return np.concatenate(out), eng.read_state(E.STATE_V)
+
+    def work(spec, runs, into, k):
+        with E.Engine.structured(spec, seed=k + 1, ou=(3.0, 0.5, 10.0), push=False, pull=True) as eng:
+            into[k] = steps(eng, runs)
+
+    runs = (400, 40)
+    alone, together = {}, {}
+    for k in (0, 1):
+        work(specs[k], runs[k], alone, k)
+    threads = [threading.Thread(target=work, args=(specs[k], runs[k], together, k)) for k in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in (0, 1):
+        assert alone[k][0].sum() > 0
+        assert all(np.array_equal(a, b) for a, b in zip(alone[k], together[k]))
+
+
 @pytest.mark.parametrize("ts", [1, 4, 255])
 def test_kernel_times_with_substeps(gpu, ts):
     """Per-kernel timing of a run with substeps and synaptic-current outputs: every launch of a step
