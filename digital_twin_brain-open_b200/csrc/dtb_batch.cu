@@ -30,7 +30,7 @@ Batch::~Batch() {
     if (stream) cudaStreamSynchronize(stream);
     if (graph) cudaGraphExecDestroy(graph);
     for (void* p : {static_cast<void*>(d_views), static_cast<void*>(d_prefix), static_cast<void*>(list),
-                    static_cast<void*>(list_count), static_cast<void*>(list_published), static_cast<void*>(local_scratch),
+                    static_cast<void*>(list_count), static_cast<void*>(list_published), static_cast<void*>(local_scratch), static_cast<void*>(pop_live),
                     static_cast<void*>(tile_net)})
         if (p) cudaFree(p);
     for (cudaEvent_t e : {ev0, ev1, tev[0], tev[1]})
@@ -106,6 +106,15 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
         DTB_CU(cudaMalloc(reinterpret_cast<void**>(&local_scratch), sizeof(uint32_t) * local_scratch_words(windows)));
         cap_windows = windows;
     }
+    uint32_t pops = 0;
+    for (const Engine* e : m) pops += e->P;
+    if (pops > cap_pops) {
+        if (pop_live) cudaFree(pop_live);
+        pop_live = nullptr;
+        DTB_CU(cudaMalloc(reinterpret_cast<void**>(&pop_live), sizeof(uint32_t) * pops));
+        cap_pops = pops;
+    }
+    DTB_CU(cudaMemsetAsync(pop_live, 0, sizeof(uint32_t) * pops, stream));
     if (!list_count) {
         DTB_CU(cudaMalloc(reinterpret_cast<void**>(&list_count), sizeof(uint32_t)));
         DTB_CU(cudaMalloc(reinterpret_cast<void**>(&list_published), 2 * sizeof(uint32_t)));
@@ -130,7 +139,8 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
     dense_min = dense_min_spikes(edges, total);
     edges_total = edges;
     windows_total = windows;
-    lb.local = LocalPlan{d_prefix + 3 * (n + 1), windows, dense_min, 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch};
+    lb.local = LocalPlan{d_prefix + 3 * (n + 1), windows, dense_min, 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch,
+                         pop_live, pops};
     lb.sm_count = static_cast<uint32_t>(sm_count);
     if (graph) {
         cudaGraphExecDestroy(graph);
@@ -145,7 +155,12 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
 
 int Batch::refresh_views() {
     std::vector<NetView> v(m.size());
-    for (size_t i = 0; i < m.size(); ++i) v[i] = m[i]->view;
+    uint32_t pops = 0;
+    for (size_t i = 0; i < m.size(); ++i) {
+        v[i] = m[i]->view;
+        v[i].pop_live = pop_live + pops;
+        pops += m[i]->P;
+    }
     DTB_CU(cudaMemcpyAsync(d_views, v.data(), sizeof(NetView) * v.size(), cudaMemcpyHostToDevice, stream));
     DTB_CU(cudaStreamSynchronize(stream));
     return DTB_OK;

@@ -247,7 +247,7 @@ LaunchBatch Engine::single_batch() const {
     b.spikes = SpikeList{list, list_count, list_published, n_pad};
     // a chosen window form takes the windows in every step, the tuner's choice in busy steps only
     b.local = LocalPlan{prefix_dev + 6, n_windows, window_always ? 1u : dense_min_spikes(n_edges, n),
-                        window_always ? 1u : 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch};
+                        window_always ? 1u : 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch, pop_live, P};
     b.sm_count = static_cast<uint32_t>(sm_count);
     return b;
 }

@@ -954,8 +954,7 @@ __device__ __forceinline__ void local_prep(const NetView* __restrict__ nets, con
         all += r;
     }
     __syncthreads();
-    for (uint32_t k = 0; k < n_nets; ++k)
-        for (uint32_t p = threadIdx.x; p < nets[k].n_pops; p += nt) nets[k].pop_live[p] = 0u;
+    for (uint32_t p = threadIdx.x; p < lp.pops; p += nt) lp.live[p] = 0u;
     if (!busy) return;
     // the unit size that spreads the step's rows over the SMs, then the windows' unit prefix
     uint32_t sum;

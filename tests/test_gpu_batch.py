@@ -98,6 +98,34 @@ def test_batch_local_push_step(gpu, graph, param):
         e.close()
 
 
+def test_batch_windows_over_a_run_give_the_solo_bits(gpu):
+    """The windows of every step over a run: each member's spiking rows are counted into the batch's own
+    array and emptied after every step, whatever the members' population counts; a member that steps
+    alone in between counts into its own."""
+    specs = _members()
+    res = []
+    for batched in (False, True):
+        engines = [E.Engine.structured(s, seed=i, ou=(0.9, 0.3, 10.0)) for i, s in enumerate(specs)]
+        for e in engines:
+            e.set_push_variant(*((E.PUSH_LOCAL, 8) if batched else (E.PUSH_REG, 8)))
+        if batched:
+            with E.Batch(engines) as b:
+                b.set_push_variant(E.PUSH_LOCAL, 2016)
+                first = b.run(250, syn_mode=E.SYN_PUSH_FIXED)
+                alone = engines[2].run(60, syn_mode=E.SYN_PUSH_FIXED)
+                last = b.run(150, syn_mode=E.SYN_PUSH_FIXED)
+        else:
+            first = [e.run(250, syn_mode=E.SYN_PUSH_FIXED) for e in engines]
+            alone = engines[2].run(60, syn_mode=E.SYN_PUSH_FIXED)
+            last = [e.run(150, syn_mode=E.SYN_PUSH_FIXED) for e in engines]
+        res.append([np.concatenate([a.freqs, z.freqs]) for a, z in zip(first, last)] + [alone.freqs] +
+                   [e.read_state(k) for e in engines for k in (E.STATE_V, E.STATE_J)])
+        for e in engines:
+            e.close()
+    assert all(f.sum() > 0 for f in res[0][:5])
+    assert all(np.array_equal(x, y) for x, y in zip(*res))
+
+
 def test_batch_rejects_mixed_weight_types(gpu):
     a = E.Engine.structured(nw.structured_spec(3000, 3, 50, 1))
     b = E.Engine.structured(nw.structured_spec(3000, 3, 50, 2), weight_type=E.W_BF16)
