@@ -323,7 +323,9 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
                     for (size_t i = 0; i < m.size(); ++i) v[i] = m[i]->view;
                     if (tune_class != (size_class << 2 | static_cast<uint32_t>(acc))) {
                         tune.reset();       // samples of another membership size or mode do not carry over
-                        tune.observe = 0;   // a batch serves requests: tune on the first busy steps
+                        // a batch serves requests: it tunes on the first busy steps, after a burst
+                        // period of reads where it has windows to weigh
+                        tune.observe = windows_total ? kTuneObserve : 0u;
                         tune.want = 2;
                         tune_class = size_class << 2 | static_cast<uint32_t>(acc);
                     }

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 #include <random>
 
 namespace dtb {
@@ -1101,26 +1102,42 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
     return DTB_OK;
 }
 
-// The variant to keep: the fastest mean, except that variants within kTuneTie of it
-// count as tied (a few sampled steps do not resolve smaller differences) and the tie
-// goes to the concurrent population-local push, then to list order.  On the regional
-// 5M network local:8 and local:2008 come within 1-3 % of each other on the sampled
-// bursts, while over whole runs local:2008 is 6.6 % faster (push 0.548 vs 0.585 ms).
+// The variant to keep.  Of the scattering forms the fastest mean over the busy samples, of the window
+// forms likewise; variants within kTuneTie of the fastest count as tied (a few sampled steps do not
+// resolve smaller differences) and the tie goes to the one that is fastest over the whole run, or to
+// list order.
+//
+// The window forms take over when the whole run gains.  The samples are busy steps, where windows
+// pay; in the steps below their threshold they scatter beside an L1 that their shared memory leaves
+// small, and every step pays the LIF kernel's count and work units (kWindowStepMs: 0.6 to 1.0 us,
+// 250k to 1M quiet neurons and batches of 16 and 64).  So both kinds are timed and weighed by how
+// often each was read.  On a 16-member batch (3.0M neurons, BF16, fixed) the busy steps alone read
+// 173 against 192 us for the windows and 117 against 105 us in a common step; over whole runs they
+// ran at 219 against 213 us a step.
 constexpr float kTuneTie = 0.02f;
-static void pick_best(TuneResult& res, uint32_t dense_min) {
+constexpr float kWindowStepMs = 0.001f;
+
+static void pick_best(TuneResult& res) {
     if (res.report.empty()) { res.best_ms = 0.0f; return; }
-    // A network whose peak stays below the windows' threshold only ever scatters: the window
-    // kernel and its preparation would cost it 1 to 2 us a step for nothing.
-    auto barred = [&](const TuneEntry& t) { return t.cfg.kind == PUSH_LOCAL && res.peak < dense_min; };
-    float fastest = 1e30f;
-    for (const TuneEntry& t : res.report)
-        if (!barred(t)) fastest = std::min(fastest, t.ms);
-    const TuneEntry* pick = nullptr;
-    for (const TuneEntry& t : res.report) {
-        if (barred(t) || t.ms > fastest * (1.0f + kTuneTie)) continue;
-        const bool preferred = t.cfg.kind == PUSH_LOCAL && t.cfg.param == kLocalConcurrent2;
-        if (!pick || (preferred && !(pick->cfg.kind == PUSH_LOCAL && pick->cfg.param == kLocalConcurrent2))) pick = &t;
-    }
+    const double f = static_cast<double>(res.dense) / std::max(1u, res.observed);
+    const bool weigh = res.quiet.size() == res.report.size();           // else every step read was of one kind
+    auto whole = [&](const TuneEntry* t) {
+        return weigh ? f * t->ms + (1.0 - f) * res.quiet[t - res.report.data()].ms : static_cast<double>(t->ms);
+    };
+    auto fastest = [&](bool local) {
+        float least = 1e30f;
+        for (const TuneEntry& t : res.report)
+            if ((t.cfg.kind == PUSH_LOCAL) == local) least = std::min(least, t.ms);
+        const TuneEntry* pick = nullptr;
+        for (const TuneEntry& t : res.report) {
+            if ((t.cfg.kind == PUSH_LOCAL) != local || t.ms > least * (1.0f + kTuneTie)) continue;
+            if (!pick || (weigh && whole(&t) < whole(pick))) pick = &t;
+        }
+        return pick;
+    };
+    const TuneEntry* pick = fastest(false);
+    const TuneEntry* local = res.dense ? fastest(true) : nullptr;       // no step reached the threshold: only scatters
+    if (local && whole(local) + kWindowStepMs < whole(pick)) pick = local;
     res.best = pick->cfg;
     res.best_ms = pick->ms;
 }
@@ -1138,15 +1155,22 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
     res.sampled = false;
     ++res.observed;
     res.peak = std::max(res.peak, count);
-    if (res.observed <= res.observe || count < res.peak / 2 || count < std::max<uint64_t>(64u, total_n / 500u)) {
+    const bool windows = acc != ACC_EXACT && b.local.windows != 0, below = count < b.local.dense_min;
+    if (below) res.quiet_spikes += count;
+    else ++res.dense;
+    const bool seen = res.observed > res.observe;
+    const bool busy = seen && res.samples < res.want && count >= res.peak / 2 && count >= std::max<uint64_t>(64u, total_n / 500u);
+    const bool common = windows && seen && res.dense && below && res.quiet.empty() &&
+                        static_cast<double>(count) * (res.observed - res.dense) >= res.quiet_spikes;
+    if (!busy && !common) {
         if (res.observed >= res.observe + kTuneGiveUp) {
             // settle: the best of the samples so far, or the default variant
             res.tuned = true;
-            pick_best(res, b.local.dense_min);
+            pick_best(res);
         }
         return DTB_OK;
     }
-    res.sampled = true;
+    res.sampled = busy;
     const size_t per = acc == ACC_EXACT ? sizeof(long long) * 4 : acc == ACC_FIXED ? sizeof(unsigned long long) * 2 : sizeof(float4);
     void* scratch = nullptr;
     NetView* tview = nullptr;
@@ -1155,10 +1179,13 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         cudaFree(scratch);
         return cuda_fail(cudaErrorMemoryAllocation, "tune_push");
     }
-    // Between replays L2 is overwritten: in a run a step's rows come from DRAM, while a replay of a
-    // step of some ten MB would find them in L2 and favour the variants with little in flight (on a
-    // 12-member batch the window form, measured warm, was kept although it ran 36 % slower).
-    // Without room for the buffer the replays run warm.
+    // Between replays L2 is overwritten and the sums are touched again: in a run a step's rows come
+    // from DRAM and its sums are where the LIF kernel has just left them.  A replay that finds the
+    // rows in L2 favours the variants with little in flight (on a 12-member batch the window form,
+    // measured warm, was kept although it ran 36 % slower); one that finds the sums in DRAM hides
+    // what sets the variants apart (16 members, a common step: windows against scatter 91 to 104
+    // against 90 to 99 us cold, 88 to 95 against 78 to 84 us so).  Without room for the buffer the
+    // replays run warm.
     constexpr size_t kFlushBytes = 192ull << 20;
     void* flush = nullptr;
     if (cudaMalloc(&flush, kFlushBytes) != cudaSuccess) {
@@ -1184,23 +1211,40 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         DTB_CU(cudaMemsetAsync(scratch, 0, per * total_n, stream));
         LaunchBatch tb = b;
         tb.nets = tview;
+        std::vector<uint32_t> ctas;
         for (const PushCfg& c : kPushCands) {
-            if (c.kind == PUSH_LOCAL && (acc == ACC_EXACT || b.local.windows == 0)) continue;
-            uint32_t ctas = 0;
-            DTB_CU(push_prepare(acc, wtype, c, sm_count, &ctas));
-            float ms_min = 1e30f;
-            for (int rep = 0; rep < 3; ++rep) {
+            if (c.kind == PUSH_LOCAL && !windows) continue;
+            uint32_t n = 0;
+            DTB_CU(push_prepare(acc, wtype, c, sm_count, &n));
+            step.push_back({c, 1e30f});
+            ctas.push_back(n);
+        }
+        // Replays go in rounds, so that a slow moment (clocks rising after the read's wait) falls on
+        // one replay of several variants, not on all of one's.  A busy step counts with the least of
+        // three; a common step is a few of the events' 2 us ticks long and counts with the mean of
+        // the lower two thirds of nine.
+        const int reps = common ? 9 : 3;
+        std::vector<std::vector<float>> ms_of(step.size());
+        for (int rep = 0; rep < reps; ++rep) {
+            for (size_t k = 0; k < step.size(); ++k) {
                 DTB_CU(reset_units());
-                if (flush) DTB_CU(cudaMemsetAsync(flush, rep, kFlushBytes, stream));
+                if (flush) {
+                    DTB_CU(cudaMemsetAsync(flush, rep, kFlushBytes, stream));
+                    DTB_CU(cudaMemsetAsync(scratch, 0, per * total_n, stream));
+                }
                 DTB_CU(cudaEventRecord(ev[0], stream));
-                DTB_CU(launch_push(tb, acc, wtype, c, ctas, stream));
+                DTB_CU(launch_push(tb, acc, wtype, step[k].cfg, ctas[k], stream));
                 DTB_CU(cudaEventRecord(ev[1], stream));
                 DTB_CU(cudaEventSynchronize(ev[1]));
                 float ms = 0.f;
                 DTB_CU(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-                ms_min = std::min(ms_min, ms);
+                ms_of[k].push_back(ms);
             }
-            step.push_back({c, ms_min});
+        }
+        for (size_t k = 0; k < step.size(); ++k) {
+            std::sort(ms_of[k].begin(), ms_of[k].end());
+            step[k].ms = ms_of[k][0];
+            if (common) res.quiet.push_back({step[k].cfg, std::accumulate(ms_of[k].begin(), ms_of[k].begin() + 6, 0.0f) / 6.0f});
         }
         DTB_CU(reset_units());
         return DTB_OK;
@@ -1211,18 +1255,21 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
     cudaFree(tview);
     if (flush) cudaFree(flush);
     if (st != DTB_OK) return st;
-    // running mean per variant over the samples
-    if (res.report.size() != step.size()) {
-        res.report = step;
-        res.samples = 1;
-    } else {
-        ++res.samples;
-        for (size_t k = 0; k < step.size(); ++k)
-            res.report[k].ms += (step[k].ms - res.report[k].ms) / static_cast<float>(res.samples);
+    if (busy) {
+        // running mean per variant over the samples
+        if (res.report.size() != step.size()) {
+            res.report = step;
+            res.samples = 1;
+        } else {
+            ++res.samples;
+            for (size_t k = 0; k < step.size(); ++k)
+                res.report[k].ms += (step[k].ms - res.report[k].ms) / static_cast<float>(res.samples);
+        }
     }
-    if (res.samples < res.want) return DTB_OK;
+    // a common step too, where some steps reach the windows' threshold and some do not
+    if (res.samples < res.want || (windows && res.quiet.empty() && res.dense && res.dense < res.observed)) return DTB_OK;
     res.tuned = true;
-    pick_best(res, b.local.dense_min);
+    pick_best(res);
     return DTB_OK;
 }
 

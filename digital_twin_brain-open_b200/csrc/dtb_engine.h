@@ -31,7 +31,7 @@ struct TuneEntry { PushCfg cfg; float ms; };
 // does not qualify is retried at the next step for kTuneEager reads, then every
 // kTuneStride steps; after kTuneGiveUp reads the tuner settles for the samples it has
 // (or the default variant) so a quiet network stops paying for the reads.
-constexpr uint32_t kTuneObserve = 50;     // plain engine; a batch uses 0 (latency-sensitive)
+constexpr uint32_t kTuneObserve = 50;     // a burst period; a batch without windows uses 0 (latency-sensitive)
 constexpr uint32_t kTuneSamples = 4;      // plain engine; a batch uses 2
 constexpr uint64_t kTuneStride = 47;
 constexpr uint32_t kTuneEager = 200;
@@ -46,7 +46,17 @@ struct TuneResult {
     uint32_t observed = 0;           // steps whose spike count was read
     uint32_t peak = 0;               // largest spike count seen
     std::vector<TuneEntry> report;   // per variant: mean time per sampled step
-    void reset() { tuned = sampled = false; samples = observed = peak = 0; report.clear(); }
+    // For the window forms, which pay in some steps and cost in the others:
+    uint32_t dense = 0;              // steps read that reach the windows' threshold
+    double quiet_spikes = 0.0;       // spikes of the steps read that do not
+    std::vector<TuneEntry> quiet;    // per variant: time of one step of those with at least their mean load
+    void reset() {
+        tuned = sampled = false;
+        samples = observed = peak = dense = 0;
+        quiet_spikes = 0.0;
+        report.clear();
+        quiet.clear();
+    }
     // run-relative step of the next call after one at step `s`
     uint64_t next_step(uint64_t s) const {
         return s + ((sampled || observed >= observe + kTuneEager) ? kTuneStride : 1);

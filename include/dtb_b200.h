@@ -237,8 +237,11 @@ int32_t dtb_info(void* engine, dtb_engine_info* info);
  * kind < 0 re-enables the autotuner.  From step 300 it reads the spike count of
  * every step for 50 steps, then times every variant on the live spike lists of
  * four steps with at least half the peak count seen (and 0.2 % of the neurons),
- * 47 or more steps apart, and keeps the variant with the smallest mean; it gives
- * up (keeping the best so far, or kind 0 param 8) after 400 reads of quiet steps. */
+ * 47 or more steps apart, and of one step with the mean load of those in which
+ * window forms scatter.  It keeps the variant with the smallest mean over the four,
+ * a window form only if it also wins when both kinds of step are weighed by how
+ * often they were read; it gives up (keeping the best so far, or kind 0 param 8)
+ * after 400 reads of quiet steps. */
 int32_t dtb_set_push_variant(void* engine, int32_t kind, int32_t param);
 /* Window graphs of dtb_run (no reference counterpart): with enable != 0 (the
  * default) a chunk of push-mode steps is launched kernel by kernel the first two

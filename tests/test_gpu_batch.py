@@ -126,6 +126,24 @@ def test_batch_windows_over_a_run_give_the_solo_bits(gpu):
     assert all(np.array_equal(x, y) for x, y in zip(*res))
 
 
+@pytest.mark.parametrize("specs,windows", [(nw.ensemble_specs(n_members=16, seed=3), False),
+                                           ([nw.structured_spec(300_000, 30, 600, seed=s) for s in range(3)], True)],
+                         ids=["uneven16", "dense3"])
+def test_batch_tuner_weighs_windows_over_the_whole_run(gpu, specs, windows):
+    """The window forms win the busiest steps of both batches by a tenth and by almost half.  In the
+    uneven ensemble, whose members burst out of step, they lose as much in the nine tenths of the steps
+    below their threshold: there the tuner keeps a scattering form, in the dense one a window form."""
+    engines = [E.Engine.structured(s, weight_type=E.W_BF16, seed=100 + i) for i, s in enumerate(specs)]
+    with E.Batch(engines) as b:
+        for _ in range(9):
+            b.run(100, syn_mode=E.SYN_PUSH_FIXED)
+        inf = b.info()
+        assert inf["graph_launches"] > 0              # tuned: the last windows were replayed
+        assert (inf["push_kind"] == E.PUSH_LOCAL) == windows
+    for e in engines:
+        e.close()
+
+
 def test_batch_rejects_mixed_weight_types(gpu):
     a = E.Engine.structured(nw.structured_spec(3000, 3, 50, 1))
     b = E.Engine.structured(nw.structured_spec(3000, 3, 50, 2), weight_type=E.W_BF16)
