@@ -168,7 +168,7 @@ struct NetView {
 struct SpikeList {
     uint32_t* list;                // virtual neuron ids: vbase[net] + neuron
     uint32_t* count;               // entries so far in the step being stepped
-    uint32_t* published;           // [0] the finished step's list length, read by the push; [1] finished networks of the launch
+    uint32_t* published;           // [0] the finished step's list length, read by the push; [1] finished tiles of the launch
     uint32_t capacity;
 };
 

@@ -309,16 +309,15 @@ __device__ __forceinline__ void lif_prefetch(const NetView* __restrict__ nets, c
 }
 
 // thread 0: the CTA finished `cnt` tiles of `nv`; the last CTA of the network advances its clock
-// (returns 1 then, else 0)
-__device__ __forceinline__ uint32_t lif_ticket(const NetView& nv, uint32_t cnt, float t, unsigned long long n) {
+__device__ __forceinline__ void lif_ticket(const NetView& nv, uint32_t cnt, float t, unsigned long long n) {
     __threadfence();
     const uint32_t k = atomicAdd(nv.ticket, cnt);
-    if (k + cnt != nv.lif_tiles) return 0u;
-    nv.clock->t = t;
-    nv.clock->n = n;
-    *nv.ticket = 0u;
-    __threadfence();
-    return 1u;
+    if (k + cnt == nv.lif_tiles) {
+        nv.clock->t = t;
+        nv.clock->n = n;
+        *nv.ticket = 0u;
+        __threadfence();
+    }
 }
 
 // A CTA steps chunks of `chunk` consecutive tiles, chunks strided by the grid:
@@ -367,7 +366,6 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     __shared__ float s_tk_t[kTicketSlots];
     __shared__ unsigned long long s_tk_n[kTicketSlots];
     uint32_t n_tk = 0;                 // thread 0's count of table entries
-    uint32_t nets_done = 0;            // networks this CTA was the last to finish (thread 0)
     if (tid < 2 * kStatSlots) { s_cnt[tid / kStatSlots][tid % kStatSlots] = 0; s_vs[tid / kStatSlots][tid % kStatSlots] = 0; }
     if (tid == 0) {
         for (int s = 0; s < kLifStages; ++s) mbar_init(&s_bar[s], 1);
@@ -392,7 +390,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
             // read-only cache, so switching needs no barrier)
             if (tid == 0 && done_here) {
                 if (n_tk == kTicketSlots) {
-                    for (uint32_t q = 0; q < n_tk; ++q) nets_done += lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
+                    for (uint32_t q = 0; q < n_tk; ++q) lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
                     n_tk = 0;
                 }
                 s_tk_net[n_tk] = cur_net;
@@ -660,17 +658,22 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     // the CTA's last stores complete before its tiles count towards the clock
     if (tid == 0) {
         bulk_wait_all();
-        for (uint32_t q = 0; q < n_tk; ++q) nets_done += lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
-        if (done_here) nets_done += lif_ticket(nets[cur_net], done_here, t_last_tile, n_last_tile);
+        for (uint32_t q = 0; q < n_tk; ++q) lif_ticket(nets[s_tk_net[q]], s_tk_cnt[q], s_tk_t[q], s_tk_n[q]);
+        if (done_here) lif_ticket(nets[cur_net], done_here, t_last_tile, n_last_tile);
     }
-    // the CTA that finishes the launch's last network hands the step's list to the push kernel,
-    // empties it for the next step, and prepares the windows' work units
+    // the CTA that finishes the launch's last tiles hands the step's list to the push kernel,
+    // empties it for the next step, and prepares the windows' work units.  A thread of another warp
+    // counts the launch's tiles, while thread 0 waits for the CTA's last stores and hands in its
+    // networks' (behind those tickets the count cost a 12-member batch's step 1 us): the list and
+    // the counts per population were complete at the last tile's barrier.
     if (flags & kFlagList) {
         __shared__ uint32_t s_warp[33];
         __shared__ uint32_t s_published;               // list length + 1 in the last CTA, else 0
-        if (tid == 0) {
+        if (tid == 32) {
             s_published = 0u;
-            if (nets_done && (n_nets == 1 || atomicAdd(sl.published + 1, nets_done) + nets_done == n_nets)) {
+            __threadfence();                           // this CTA's entries before its tiles
+            if (atomicAdd(sl.published + 1, it) + it == total_tiles) {
+                __threadfence();                       // the other CTAs' tiles before their entries
                 const uint32_t c = __ldcg(sl.count);
                 sl.published[0] = c;
                 sl.published[1] = 0u;
