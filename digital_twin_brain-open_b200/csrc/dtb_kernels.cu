@@ -664,7 +664,7 @@ lif_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ tile_p
     // the CTA that finishes the launch's last tiles hands the step's list to the push kernel,
     // empties it for the next step, and prepares the windows' work units.  A thread of another warp
     // counts the launch's tiles, while thread 0 waits for the CTA's last stores and hands in its
-    // networks' (behind those tickets the count cost a 12-member batch's step 1 us): the list and
+    // networks' (behind those tickets the count cost a step 0.2 us, a batch of 64 networks 1.2 us): the list and
     // the counts per population were complete at the last tile's barrier.
     if (flags & kFlagList) {
         __shared__ uint32_t s_warp[33];
@@ -768,15 +768,14 @@ __device__ __forceinline__ void push_span(const uint32_t* col, const void* wts, 
 // per warp, for short rows).  With fewer rows than groups of lanes, a row is cut into
 // interleaved parts of U x LPR synapses so that a quiet step (a few dozen rows, most of the
 // steps of a bursting network) is one round of loads deep instead of one per U x LPR synapses.
-template <int ACC, int WT, int U, int LPR>
+template <int ACC, int WT, int U, int LPR, bool CUT>
 __device__ __forceinline__ void push_rows(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets,
-                                          const SpikeList& sl, uint32_t count) {
+                                          const SpikeList& sl, uint32_t count, uint32_t cut) {
     constexpr uint32_t kGroups = 32 / LPR;
-    constexpr uint32_t kMaxParts = 8;
     const uint32_t lane = (threadIdx.x & 31u) % LPR;
     const uint32_t gw = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kGroups + (threadIdx.x & 31u) / LPR;
     const uint32_t nw = ((gridDim.x * blockDim.x) >> 5) * kGroups;
-    const uint32_t parts = count ? min(kMaxParts, max(1u, nw / count)) : 1u;
+    const uint32_t parts = CUT ? cut : 1u;
     const uint32_t total = count * parts;            // below nw, or count itself
     const uint32_t* col = nets[0].out_col;
     const void* wts = nets[0].out_w;
@@ -785,7 +784,7 @@ __device__ __forceinline__ void push_rows(const NetView* __restrict__ nets, cons
     const unsigned long long keep = l2_policy_keep();
     uint32_t vb = 0;
     for (uint32_t r = gw; r < total; r += nw) {
-        const uint32_t row = parts > 1 ? r / parts : r, part = r - row * parts;
+        const uint32_t row = CUT ? r / parts : r, part = r - row * parts;
         const uint32_t v = __ldg(sl.list + row);
         if (n_nets > 1) {
             const uint32_t k = find_net(vbase, n_nets, v);
@@ -802,10 +801,21 @@ __device__ __forceinline__ void push_rows(const NetView* __restrict__ nets, cons
     }
 }
 
+// The number of parts is settled once: the loop over whole rows keeps a constant stride.
+template <int ACC, int WT, int U, int LPR>
+__device__ __forceinline__ void push_list(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets,
+                                          const SpikeList& sl, uint32_t count) {
+    constexpr uint32_t kMaxParts = 8;
+    const uint32_t nw = ((gridDim.x * blockDim.x) >> 5) * (32 / LPR);
+    const uint32_t parts = count ? min(kMaxParts, nw / count) : 1u;
+    if (parts > 1) push_rows<ACC, WT, U, LPR, true>(nets, vbase, n_nets, sl, count, parts);
+    else push_rows<ACC, WT, U, LPR, false>(nets, vbase, n_nets, sl, count, 1u);
+}
+
 template <int ACC, int WT, int U, int LPR>
 __global__ void __launch_bounds__(kPushThreads)
 push_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ vbase, uint32_t n_nets, SpikeList sl) {
-    push_rows<ACC, WT, U, LPR>(nets, vbase, n_nets, sl, *sl.published);
+    push_list<ACC, WT, U, LPR>(nets, vbase, n_nets, sl, *sl.published);
 }
 
 // ---------------------------------------------------------------------------
@@ -1208,7 +1218,7 @@ push_window_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict_
     const uint32_t count = *sl.published;
     const uint32_t total_units = lp.scratch[2 * lp.windows];
     if (total_units == 0) {
-        push_rows<ACC, WT, 8, 32>(nets, vbase, n_nets, sl, count);
+        push_list<ACC, WT, 8, 32>(nets, vbase, n_nets, sl, count);
     } else {
         if (threadIdx.x < win_threads)
             push_windows<WT, RLW, ACC == ACC_FIXED>(nets, lp, n_nets, total_units, acc, s_warp, &s_unit, win_threads);
