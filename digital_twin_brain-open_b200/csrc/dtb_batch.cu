@@ -138,6 +138,7 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
     for (const Engine* e : m) edges += e->n_edges;
     dense_min = dense_min_spikes(edges, total);
     edges_total = edges;
+    lb.pull_degree = static_cast<uint32_t>(edges / std::max<uint64_t>(1u, total));
     windows_total = windows;
     lb.local = LocalPlan{d_prefix + 3 * (n + 1), windows, dense_min, 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch,
                          pop_live, pops};

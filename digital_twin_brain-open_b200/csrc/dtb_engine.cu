@@ -242,6 +242,7 @@ LaunchBatch Engine::single_batch() const {
     b.n_nets = 1;
     b.lif_tiles_total = n_pad / kLifTile;
     b.pull_tiles_total = n_pad / kPullTile;
+    b.pull_degree = static_cast<uint32_t>(n_edges / std::max(1u, n));
     b.push_ctas = static_cast<uint32_t>(sm_count) * 8u;
     b.lif_ctas = static_cast<uint32_t>(sm_count) * lif_ctas_per_sm;
     b.lif_chunk = 1;

@@ -2048,10 +2048,19 @@ static void pull_dispatch(const LaunchBatch& b, int wt, uint32_t flags, int prop
     }
 }
 
+// In-edges a neuron from which the bitmap goes to shared memory.  That form keeps 16 edges in flight
+// per lane and one CTA per SM, so it needs rows of half a round (16 x 32) or more; shorter ones leave
+// its lanes idle and its one CTA short of rows.  Measured, shared memory against L2, FP32, us a step:
+// 20,000 neurons 39 / 31 with 100 edges, 58 / 58 with 200, 74 / 86 with 300, 51 / 77 with 400;
+// 200,000 neurons 107 / 77, 189 / 192, 226 / 250, 201 / 256, and 221 / 357 with 1,000; 500,000
+// neurons 247 / 157, 442 / 375, 501 / 474, 398 / 475.  BF16: 93 / 57 with 60, 220 / 253 with 400
+// (200,000 neurons).
+constexpr uint32_t kPullSmemDegree = 256;
+
 // Whether a launch's bitmap goes to shared memory, and the bytes it takes (0: it stays in L2).
 static uint32_t pull_smem_bytes(const LaunchBatch& b) {
     const uint32_t neurons = b.pull_tiles_total * kPullTile;
-    if (b.n_nets != 1 || neurons > kPullSmemNeurons) return 0;
+    if (b.n_nets != 1 || neurons > kPullSmemNeurons || b.pull_degree < kPullSmemDegree) return 0;
     return (neurons + kPad - 1) / kPad * kPad / 8;
 }
 

@@ -49,6 +49,7 @@ struct LaunchBatch {
     uint32_t n_nets;
     uint32_t lif_tiles_total;
     uint32_t pull_tiles_total;
+    uint32_t pull_degree;         // mean in-edges of a neuron
     uint32_t push_ctas;
     uint32_t lif_ctas;            // persistent grid of the LIF kernel
     uint32_t lif_chunk;           // consecutive tiles a LIF CTA steps before striding (0 or 1: one)

@@ -62,10 +62,11 @@ def test_da_filter_ragged(gpu, members, voxels, hp):
     assert np.allclose(out.cpu().numpy(), da_filter(w, y, noise, hp, 1e-3, 0.3), rtol=2.5e-7, atol=1e-7)
 
 
-@pytest.mark.parametrize("n,pops,degree", [(31, 1, 5), (1025, 3, 17), (40_003, 9, 700), (1_700_001, 5, 20)])
+@pytest.mark.parametrize("n,pops,degree", [(31, 1, 5), (31, 1, 300), (1025, 3, 17), (1025, 3, 257), (40_003, 9, 255), (40_003, 9, 700),
+                                           (1_638_400, 5, 256), (1_700_001, 5, 20)])
 def test_pull_equals_exact_push(gpu, n, pops, degree):
-    """The pull's 64-bit sums equal the exact push's bit for bit; 1.7M neurons' bitmap is too large
-    for shared memory."""
+    """The pull's 64-bit sums equal the exact push's bit for bit, from 256 in-edges a neuron on with the
+    bitmap in shared memory (1,638,400 neurons fill it), below and above that size in L2."""
     spec = nw.structured_spec(n, pops, degree, seed=n, min_pop=8)
     res = []
     for syn in (E.SYN_PUSH_EXACT, E.SYN_PULL):
@@ -80,10 +81,10 @@ def test_pull_equals_exact_push(gpu, n, pops, degree):
 
 
 def test_pulls_of_two_sizes_from_two_threads(gpu):
-    """Two threads step a small network and one with the largest bitmap that shared memory takes:
-    each gives the bits it gives alone."""
+    """Two threads step a small network and one whose bitmap is over shared memory's default limit (both
+    with their bitmaps there): each gives the bits it gives alone."""
     import threading
-    specs = [nw.structured_spec(n, 3, 5, seed=n) for n in (2_000, 1_638_400)]
+    specs = [nw.structured_spec(n, 3, 256, seed=n) for n in (2_000, 600_000)]
 
     def steps(eng, runs):
         out = [eng.run(3, syn_mode=E.SYN_PULL).freqs for _ in range(runs)]
