@@ -100,32 +100,25 @@ da_stats_kernel(uint32_t E, uint32_t V, uint32_t S, uint32_t vb, uint32_t width,
     }
 }
 
-// G[e][f] = sum_v I[e,v] T[f,v] / V.  A CTA makes an 8 x 8 tile: rows of 256 voxels of both
-// factors are staged in shared memory and four threads share a product's voxels (a warp per
-// product re-read both rows for each of the E^2 products).
-constexpr int kGainTile = 8, kGainVox = 256;
-__global__ void __launch_bounds__(kDaThreads)
+// G[e][f] = sum_v I[e,v] T[f,v] / V: one warp per (e, f).  The factors are read from L2 for each of
+// the E^2 products; 8 x 8 tiles of products that staged them in shared memory measured slower at
+// every size (whole filter: 16 x 3000 x 6 34 against 66 us, 100 x 1000 x 10 64 against 78, 150 x
+// 3000 x 16 289 against 360), each tile being a chain over all voxels on few CTAs.  Count holds E^2.
+template <class Count>
+__global__ void __launch_bounds__(256)
 da_gain_kernel(uint32_t E, uint32_t V, const double* __restrict__ innov, const double* __restrict__ temp,
                double* __restrict__ gain) {
-    __shared__ double s_i[kGainTile][kGainVox + 1], s_t[kGainTile][kGainVox + 1];
-    const uint32_t tiles = (E + kGainTile - 1) / kGainTile;
-    const uint32_t e0 = blockIdx.x / tiles * kGainTile, f0 = blockIdx.x % tiles * kGainTile;
-    const uint32_t part = threadIdx.x & 3u, pair = threadIdx.x >> 2, e = pair / kGainTile, f = pair % kGainTile;
-    double acc = 0.0;
-    for (uint32_t v0 = 0; v0 < V; v0 += kGainVox) {
-        __syncthreads();
-        for (uint32_t k = threadIdx.x; k < kGainTile * kGainVox; k += kDaThreads) {
-            const uint32_t r = k / kGainVox, v = v0 + k % kGainVox;
-            s_i[r][k % kGainVox] = v < V && e0 + r < E ? innov[static_cast<size_t>(e0 + r) * V + v] : 0.0;
-            s_t[r][k % kGainVox] = v < V && f0 + r < E ? temp[static_cast<size_t>(f0 + r) * V + v] : 0.0;
-        }
-        __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    const Count products = static_cast<Count>(E) * E;
+    for (Count k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < products; k += nw) {
+        const uint32_t e = static_cast<uint32_t>(k / E), f = static_cast<uint32_t>(k % E);
+        double acc = 0.0;
+        for (uint32_t v = lane; v < V; v += 32) acc += innov[static_cast<size_t>(e) * V + v] * temp[static_cast<size_t>(f) * V + v];
 #pragma unroll
-        for (uint32_t k = part; k < kGainVox; k += 4) acc = __fma_rn(s_i[e][k], s_t[f][k], acc);
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) gain[k] = acc / V;
     }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    if (part == 0 && e0 + e < E && f0 + f < E) gain[static_cast<size_t>(e0 + e) * E + f0 + f] = acc / V;
 }
 
 // Update: a thread owns one column (voxel, state) for kUpdRows members, so a deviation is read
@@ -198,8 +191,9 @@ extern "C" int32_t dtb_da_filter(uint32_t ensembles, uint32_t voxels, uint32_t s
     while (width < vb * S && width < dtb::kDaThreads) width *= 2;
     dtb::da_stats_kernel<<<static_cast<uint32_t>((V + vb - 1) / vb), dtb::kDaThreads, 0, s>>>(
         ensembles, voxels, states, vb, width, w_hat, bold_y, noise, bold_sigma, mean, temp, innov, colsum);
-    const uint32_t tiles = (ensembles + dtb::kGainTile - 1) / dtb::kGainTile;
-    dtb::da_gain_kernel<<<tiles * tiles, dtb::kDaThreads, 0, s>>>(ensembles, voxels, innov, temp, gain);
+    const uint32_t gain_ctas = static_cast<uint32_t>(std::min<size_t>((E * E + 7) / 8, 4096));
+    if (E < 65536) dtb::da_gain_kernel<uint32_t><<<gain_ctas, 256, 0, s>>>(ensembles, voxels, innov, temp, gain);
+    else dtb::da_gain_kernel<unsigned long long><<<gain_ctas, 256, 0, s>>>(ensembles, voxels, innov, temp, gain);
     const dim3 grid(static_cast<uint32_t>((V * S + dtb::kUpdThreads - 1) / dtb::kUpdThreads), (ensembles + dtb::kUpdRows - 1) / dtb::kUpdRows);
     dtb::da_update_kernel<<<grid, dtb::kUpdThreads, 0, s>>>(ensembles, voxels, states, w_hat, mean, innov, colsum, gain, rate, w_out);
     e = cudaGetLastError();
