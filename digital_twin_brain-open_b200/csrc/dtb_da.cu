@@ -185,8 +185,18 @@ extern "C" int32_t dtb_da_filter(uint32_t ensembles, uint32_t voxels, uint32_t s
     double* temp = colsum + n_mean;
     double* innov = temp + n_ev;
     double* gain = innov + n_ev;
-    // voxels per statistics CTA: as many as fill its threads once over, down to one
-    const uint32_t vb = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(64 / S, V)));
+    int dev = 0, sms = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) {
+        cudaFreeAsync(buf, s);
+        return dtb::cuda_fail(e, "dtb_da_filter");
+    }
+    // voxels per statistics CTA: as many as 64 columns take, fewer where that leaves an SM fewer than
+    // two CTAs (a narrower CTA also walks the members in fewer turns).  Whole filter, 64 columns
+    // against this: 150 x 50 x 6 60 / 40 us, 64 x 300 x 6 37 / 30, 16 x 1000 x 6 27 / 25; four or
+    // eight CTAs an SM cost the last 2 and 7 us more.
+    const uint32_t vb = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(64 / S, (V + 2 * sms - 1) / (2 * sms))));
     uint32_t width = 1;
     while (width < vb * S && width < dtb::kDaThreads) width *= 2;
     dtb::da_stats_kernel<<<static_cast<uint32_t>((V + vb - 1) / vb), dtb::kDaThreads, 0, s>>>(

@@ -50,7 +50,8 @@ def test_bold_remainders_and_powers(gpu, n, steps, alpha):
     assert np.allclose(st.cpu().numpy(), o.state(), rtol=2e-6, atol=1e-7)
 
 
-@pytest.mark.parametrize("members,voxels,hp", [(2, 1, 0), (3, 7, 1), (33, 65, 4), (101, 64, 10), (129, 130, 58), (16, 5, 300)])
+@pytest.mark.parametrize("members,voxels,hp", [(2, 1, 0), (3, 7, 1), (33, 65, 4), (101, 64, 10), (129, 130, 58), (16, 5, 300),
+                                               (20, 1000, 4), (7, 700, 0), (151, 300, 0)])
 def test_da_filter_ragged(gpu, members, voxels, hp):
     import torch
     rng = np.random.default_rng(members * 1000 + hp)
