@@ -124,7 +124,11 @@ da_gain_kernel(uint32_t E, uint32_t V, const double* __restrict__ innov, const d
 // Update: a thread owns one column (voxel, state) for kUpdRows members, so a deviation is read
 // and widened once for kUpdRows products (one thread per output widened it for each); the
 // members' gains sit in shared memory and are read as broadcasts, kUpdChunk of them at a time.
-constexpr int kUpdThreads = 128, kUpdRows = 10, kUpdChunk = 128;
+// Over 16 to 150 members, 1,000 and 3,000 voxels and 6 to 16 states ten members a thread run within
+// 5 us of the better of 8 and 16 and mostly are the best (150 x 3000 x 16: 8 / 10 / 16 members 297 /
+// 284 / 334 us, 97 x 3000 x 10 106 / 101 / 114, 33 x 3000 x 6 39 / 41 / 43).
+constexpr int kUpdThreads = 128, kUpdChunk = 128;
+template <int kUpdRows>
 __global__ void __launch_bounds__(kUpdThreads)
 da_update_kernel(uint32_t E, uint32_t V, uint32_t S, const float* __restrict__ w, const double* __restrict__ mean,
                  const double* __restrict__ innov, const double* __restrict__ colsum, const double* __restrict__ gain,
@@ -204,8 +208,15 @@ extern "C" int32_t dtb_da_filter(uint32_t ensembles, uint32_t voxels, uint32_t s
     const uint32_t gain_ctas = static_cast<uint32_t>(std::min<size_t>((E * E + 7) / 8, 4096));
     if (E < 65536) dtb::da_gain_kernel<uint32_t><<<gain_ctas, 256, 0, s>>>(ensembles, voxels, innov, temp, gain);
     else dtb::da_gain_kernel<unsigned long long><<<gain_ctas, 256, 0, s>>>(ensembles, voxels, innov, temp, gain);
-    const dim3 grid(static_cast<uint32_t>((V * S + dtb::kUpdThreads - 1) / dtb::kUpdThreads), (ensembles + dtb::kUpdRows - 1) / dtb::kUpdRows);
-    dtb::da_update_kernel<<<grid, dtb::kUpdThreads, 0, s>>>(ensembles, voxels, states, w_hat, mean, innov, colsum, gain, rate, w_out);
+    // ten members a thread, two where ten leave SMs without a CTA (whole filter, ten against two:
+    // 40 x 50 x 10 25 / 18 us, 100 x 50 x 6 31 / 24, 16 x 300 x 10 21 / 18)
+    const uint32_t col_ctas = static_cast<uint32_t>((V * S + dtb::kUpdThreads - 1) / dtb::kUpdThreads);
+    auto update = [&](auto kernel, uint32_t rows) {
+        kernel<<<dim3(col_ctas, (ensembles + rows - 1) / rows), dtb::kUpdThreads, 0, s>>>(ensembles, voxels, states, w_hat, mean, innov,
+                                                                                      colsum, gain, rate, w_out);
+    };
+    if (static_cast<size_t>(col_ctas) * ((E + 9) / 10) < static_cast<size_t>(sms)) update(dtb::da_update_kernel<2>, 2);
+    else update(dtb::da_update_kernel<10>, 10);
     e = cudaGetLastError();
     cudaFreeAsync(buf, s);
     if (e != cudaSuccess) return dtb::cuda_fail(e, "dtb_da_filter");
