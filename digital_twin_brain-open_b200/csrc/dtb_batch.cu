@@ -138,6 +138,8 @@ int Batch::set_members(Engine* const* engines, uint32_t n) {
     for (const Engine* e : m) edges += e->n_edges;
     dense_min = dense_min_spikes(edges, total);
     edges_total = edges;
+    neurons_total = 0;
+    for (const Engine* e : m) neurons_total += e->n;
     lb.pull_degree = static_cast<uint32_t>(edges / std::max<uint64_t>(1u, total));
     windows_total = windows;
     lb.local = LocalPlan{d_prefix + 3 * (n + 1), windows, dense_min, 0u, static_cast<uint32_t>(sm_count) * kUnitsPerSm, 1u, local_scratch,
@@ -231,7 +233,7 @@ int Batch::run(const dtb_run_request& rq, dtb_run_output* outs) {
             size_class = 64u - static_cast<uint32_t>(__builtin_clzll(total | 1ull));
             const auto it = tuned_by_size[acc].find(size_class);
             push_tuned[acc] = it != tuned_by_size[acc].end();
-            if (push_tuned[acc]) push_cfg = it->second;
+            push_cfg = push_tuned[acc] ? it->second : default_push(edges_total, neurons_total);
         }
         lb.local.dense_min = window_always ? 1u : dense_min;
         lb.local.always = window_always ? 1u : 0u;
@@ -436,6 +438,7 @@ int32_t dtb_batch_set_push_variant(void* batch, int32_t kind, int32_t param) {
     if (kind < 0) {
         b->autotune = true;
         b->window_always = false;
+        b->push_cfg = dtb::default_push(b->edges_total, b->neurons_total);
         for (int a = 0; a < 3; ++a) {
             b->push_tuned[a] = false;
             b->tuned_by_size[a].clear();

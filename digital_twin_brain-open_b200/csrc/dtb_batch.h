@@ -35,7 +35,7 @@ public:
     uint32_t cap_tiles = 0;
     uint32_t cap_windows = 0;         // capacity of local_scratch (windows)
     uint32_t windows_total = 0;       // windows of the current membership
-    uint64_t edges_total = 0;         // synapses of the current membership
+    uint64_t edges_total = 0, neurons_total = 0;   // synapses and neurons of the current membership
     uint32_t dense_min = 1;           // spikes from which a tuned window push takes the windows
     LaunchBatch lb{};
     PushCfg push_cfg{PUSH_REG, 8, 32};

@@ -555,6 +555,7 @@ int Engine::create_from_arrays(const dtb_network_arrays& a, const dtb_options& o
     DTB_TRY(upload_params());
     DTB_TRY(init_state());
     DTB_TRY(build_local_tables());
+    push_cfg = default_push(n_edges, n);
     return refresh_view();
 }
 
@@ -631,6 +632,7 @@ int Engine::create_structured(const dtb_structured_spec& s, const dtb_options& o
     DTB_TRY(upload_params());
     DTB_TRY(init_state());
     DTB_TRY(build_local_tables());
+    push_cfg = default_push(n_edges, n);
     return refresh_view();
 }
 
@@ -1753,6 +1755,7 @@ int32_t dtb_set_push_variant(void* engine, int32_t kind, int32_t param) {
     if (kind < 0) {
         e->autotune = true;
         e->window_always = false;
+        e->push_cfg = dtb::default_push(e->n_edges, e->n);     // a network that is not tuned keeps it
         for (int a = 0; a < 3; ++a) {
             e->push_tuned[a] = false;
             e->tune_acc[a].reset();

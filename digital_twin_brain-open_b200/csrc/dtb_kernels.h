@@ -70,6 +70,14 @@ struct PushCfg {
     int lpr = 32;  // PUSH_REG: lanes per row (32, 16, 8; sub-warp rows use 8 in flight per lane)
 };
 
+// The variant of a network (or batch) that is not tuned, or not yet: a warp per row, or a quarter
+// warp for rows that would leave most of a warp idle.  Eight synapses in flight by 32 against by 8
+// lanes: 32.1 / 30.1 us a step with 15 synapses a row (1M neurons, 1.1 % of them spiking), 37.1 /
+// 34.9 with 10 (1.5M), 45.8 / 43.5 with 5 (2M), 24.6 / 24.6 with 30 (500,000) and 18.5 / 18.5 with
+// 50 (300,000).
+constexpr uint64_t kShortRow = 24;
+inline PushCfg default_push(uint64_t edges, uint64_t neurons) { return PushCfg{PUSH_REG, 8, edges < kShortRow * neurons ? 8 : 32}; }
+
 // Every variant the autotuner times.
 constexpr int kPushCandidates = 12;
 // PUSH_LOCAL params: 8 (and 8 with 16 lanes per cross-population row) give every warp to the

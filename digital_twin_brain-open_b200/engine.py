@@ -368,7 +368,8 @@ class Engine:
 
     def set_push_variant(self, kind, param=0):
         """kind 0: register-staged (param 4/8/16, 1016/1008 sub-warp rows), 1: TMA-staged
-        (param 256/512), 2: population-local windows (param 8/1016), -1: autotune."""
+        (param 256/512), 2: population-local windows in every step (param 8, 1016, 2008, 2016,
+        3008), -1: autotune."""
         _check(LIB.dtb_set_push_variant(self._h, kind, param))
 
     def set_graph(self, enable):

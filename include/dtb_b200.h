@@ -240,8 +240,11 @@ int32_t dtb_info(void* engine, dtb_engine_info* info);
  * 47 or more steps apart, and of one step with the mean load of those in which
  * window forms scatter.  It keeps the variant with the smallest mean over the four,
  * a window form only if it also wins when both kinds of step are weighed by how
- * often they were read; it gives up (keeping the best so far, or kind 0 param 8)
- * after 400 reads of quiet steps. */
+ * often they were read; it gives up (keeping the best so far, or the default)
+ * after 400 reads of quiet steps.  The default, also after kind < 0 until a variant
+ * is chosen, is kind 0 with param 8, or 1008 where rows hold fewer than 24 synapses
+ * on average.  Networks of fewer than 16,000,000 synapses are not timed and keep it:
+ * a step of theirs never takes windows, and the other forms are within 5 % of it. */
 int32_t dtb_set_push_variant(void* engine, int32_t kind, int32_t param);
 /* Window graphs of dtb_run (no reference counterpart): with enable != 0 (the
  * default) a chunk of push-mode steps is launched kernel by kernel the first two

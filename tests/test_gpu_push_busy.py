@@ -85,3 +85,30 @@ def test_few_long_rows_are_cut_into_parts(gpu, out_degree):
             r = eng.run(1, use_ou=False, syn_mode=syn)
             assert r.freqs.sum() == 3 and r.events == pre.size
             assert np.array_equal(eng.read_state(E.STATE_J), ref.astype(np.float32))    # dyadic weights: exact in any order
+
+
+@pytest.mark.parametrize("degree,param", [(10, 1008), (23, 1008), (24, 8), (60, 8)])
+def test_untuned_networks_return_to_their_default_form(gpu, degree, param):
+    """A network too small to be tuned, alone and in a batch: autotuning again takes back a form chosen
+    before, rows of few synapses have the quarter-warp form, and every form gives the same bits."""
+    spec = nw.structured_spec(3000, 3, degree, seed=degree)
+    res = []
+    with E.Engine.structured(spec, seed=2, ou=(3.0, 0.5, 10.0)) as eng:
+        blob = eng.save_state()
+        for variant in (None, (E.PUSH_TMA, 512), (-1, 0)):
+            if variant is not None:
+                eng.set_push_variant(*variant)
+                eng.load_state(blob)
+            r = eng.run(400, syn_mode=E.SYN_PUSH_EXACT)
+            inf = eng.info()
+            res.append((r.freqs, r.events, eng.read_state(E.STATE_J)))
+            assert (inf.push_kind, inf.push_param) == ((E.PUSH_REG, param) if variant in (None, (-1, 0)) else variant)
+        with E.Batch([eng]) as b:
+            b.set_push_variant(E.PUSH_TMA, 512)
+            b.run(5)
+            b.set_push_variant(-1)
+            b.run(5)
+            assert (b.info()["push_kind"], b.info()["push_param"]) == (E.PUSH_REG, param)
+    assert res[0][0].sum() > 0
+    for other in res[1:]:
+        assert np.array_equal(res[0][0], other[0]) and res[0][1] == other[1] and np.array_equal(res[0][2], other[2])
