@@ -35,10 +35,10 @@ def test_compaction_edges(gpu, n, offset):
     assert bool((idx[c:] == -1).all())
 
 
-@pytest.mark.parametrize("alpha", [0.2, 0.32, 1.0, 0.5])
+@pytest.mark.parametrize("alpha", [0.2, 0.32, 1.0, 0.5, 1 / 8, 1 / 16, 1 / 17])
 @pytest.mark.parametrize("n,steps", [(1, 1), (63, 3), (65, 4), (130, 6), (257, 203)])
 def test_bold_remainders_and_powers(gpu, n, steps, alpha):
-    """Whole 1/alpha takes products, any other takes powf; both within 2e-6 of the float32 oracle,
+    """Whole 1/alpha up to 16 takes products, any other takes powf; both within 2e-6 of the float32 oracle,
     the difference of a few roundings per step (as in the BOLD tests)."""
     import torch
     u = bold_inputs(n, steps, steps + n)
