@@ -24,13 +24,26 @@ def _run(spec, variant, steps, wt, chunk=100):
         return np.concatenate(freqs), events, eng.read_state(E.STATE_V), eng.read_state(E.STATE_J), eng.info()
 
 
-@pytest.mark.parametrize("n,pops,degree,wt", [(60_011, 7, 600, E.W_F32), (90_000, 40, 400, E.W_BF16)])
+@pytest.mark.parametrize("n,pops,degree,wt", [(150_011, 9, 900, E.W_F32), (120_000, 12, 900, E.W_BF16)])
 def test_tuned_window_form_gives_the_register_pushs_bits(gpu, n, pops, degree, wt):
-    spec = nw.structured_spec(n, pops, degree, seed=31)
-    f0, e0, v0, j0, _ = _run(spec, (E.PUSH_REG, 8), 1000, wt)
-    f1, e1, v1, j1, inf = _run(spec, None, 1000, wt)              # autotuned
-    f2, e2, v2, j2, _ = _run(spec, (E.PUSH_LOCAL, 2016), 1000, wt)   # windows in every step
-    assert f0.sum(1).max() > 0.1 * n and np.median(f0.sum(1)) < 0.01 * n     # quiet steps and bursts
+    """The tuner's window form through quiet steps, busy ones, and the populations of a busy step that
+    do not pay for their windows: two populations with almost no recurrent input fire a few neurons a
+    step, in bursts of the others too, and are scattered whole while those take their windows."""
+    g_scale = np.ones((pops, 4), np.float32)
+    g_scale[:2] = 0.01
+    spec = nw.structured_spec(n, pops, degree, seed=31, g_scale=g_scale)
+    f0, e0, v0, j0, inf0 = _run(spec, (E.PUSH_REG, 8), 1500, wt)
+    f1, e1, v1, j1, inf = _run(spec, None, 1500, wt)              # autotuned
+    f2, e2, v2, j2, _ = _run(spec, (E.PUSH_LOCAL, 2016), 1500, wt)   # windows in every step
+    assert inf.push_kind == E.PUSH_LOCAL
+    busy = f0.sum(1) >= 16_000_000 * n / inf0.n_edges             # the steps in which that form takes windows
+    late = np.arange(len(f0)) >= 1000                             # well after it was chosen
+    assert 10 <= (busy & late).sum() < late.sum() // 2
+    # rows from which a window pays: (4 events a neuron + 8192) over the own-population synapses of a row
+    least = (4 * spec.pop_sizes + 8192) / (0.7 * degree)
+    cold = (f0[busy & late][:, :2] > 0) & (f0[busy & late][:, :2] < 0.5 * least[:2])
+    hot = f0[busy & late][:, 2:] > 2 * least[2:]
+    assert cold.mean() > 0.25 and hot.mean() > 0.3
     for f, e, v, j in ((f1, e1, v1, j1), (f2, e2, v2, j2)):
         assert np.array_equal(f0, f) and e0 == e
         assert np.array_equal(v0, v) and np.array_equal(j0, j)

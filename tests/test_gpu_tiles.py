@@ -51,7 +51,7 @@ def test_window_push_at_scale_gives_the_same_bits(gpu):
     """The population-window push at scale: a 1.2M-neuron regional network (24 populations of
     ~50k neurons, in-degree 300, BF16) has ~4 windows per population, and a burst step hands each
     window dozens of 1024-row work units.  With the fixed-point push the window form (local:2016,
-    its cross-population part on a second stream) and the register push must give the same bits:
+    half of each CTA's warps on the cross-population part) and the register push must give the same bits:
     per-step counts, events, V and J after 600 steps."""
     spec = nw.structured_spec(1_200_000, 24, 300, seed=8)
     results = []
