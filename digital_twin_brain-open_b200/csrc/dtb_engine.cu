@@ -1187,11 +1187,14 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
     // rows in L2 favours the variants with little in flight (on a 12-member batch the window form,
     // measured warm, was kept although it ran 36 % slower); one that finds the sums in DRAM hides
     // what sets the variants apart (16 members, a common step: windows against scatter 91 to 104
-    // against 90 to 99 us cold, 88 to 95 against 78 to 84 us so).  Without room for the buffer the
-    // replays run warm.
+    // against 90 to 99 us cold, 88 to 95 against 78 to 84 us so).  The buffer is taken only while
+    // eight of its size are free, so that a run does not take the memory another thread is about to
+    // allocate; the replays run warm without it.
     constexpr size_t kFlushBytes = 192ull << 20;
     void* flush = nullptr;
-    if (cudaMalloc(&flush, kFlushBytes) != cudaSuccess) {
+    size_t free_bytes = 0, all_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess ||
+        (free_bytes >= 8 * kFlushBytes && cudaMalloc(&flush, kFlushBytes) != cudaSuccess)) {
         cudaGetLastError();
         flush = nullptr;
     }
