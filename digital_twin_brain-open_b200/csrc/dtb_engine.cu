@@ -1105,9 +1105,11 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
     return DTB_OK;
 }
 
-// The variant to keep.  Of the scattering forms the fastest mean over the busy samples, of the window
-// forms likewise; variants within kTuneTie of the fastest count as tied (a few sampled steps do not
-// resolve smaller differences) and the tie goes to the one that is fastest over the whole run, or to
+// The variant to keep.  Of the scattering forms the fastest mean over the busy samples, unless eight
+// synapses in flight on a warp per row come within kTuneDefault of it: a few replays, away from the
+// LIF launches around them, do not resolve less (on a 12-member batch they put sixteen in flight 2 to
+// 4 % ahead, which ran 159.6 against 157.8 us a step).  Of the window forms likewise the fastest;
+// those within kTuneTie of it count as tied and the tie goes to the fastest over the whole run, or to
 // list order.
 //
 // The window forms take over when the whole run gains.  The samples are busy steps, where windows
@@ -1116,11 +1118,16 @@ int Engine::run(const dtb_run_request& rq, dtb_run_output& out) {
 // 250k to 1M quiet neurons and batches of 16 and 64).  So both kinds are timed and weighed by how
 // often each was read.  On a 16-member batch (3.0M neurons, BF16, fixed) the busy steps alone read
 // 173 against 192 us for the windows and 117 against 105 us in a common step; over whole runs they
-// ran at 219 against 213 us a step.
+// ran at 219 against 213 us a step.  In a batch, whose members burst out of step, the common steps
+// carry most of the run, and one of them replayed is up to 8 us off what the run shows (twelve
+// members, ten seeds: two read the windows 1 to 3 % ahead, which ran 3 to 5 % behind), so there the
+// windows must win by kTuneBatch (three dense members read 38 % and run 26 % ahead).
 constexpr float kTuneTie = 0.02f;
+constexpr float kTuneDefault = 0.04f;
+constexpr float kTuneBatch = 0.05f;
 constexpr float kWindowStepMs = 0.001f;
 
-static void pick_best(TuneResult& res) {
+static void pick_best(TuneResult& res, uint32_t n_nets) {
     if (res.report.empty()) { res.best_ms = 0.0f; return; }
     const double f = static_cast<double>(res.dense) / std::max(1u, res.observed);
     const bool weigh = res.quiet.size() == res.report.size();           // else every step read was of one kind
@@ -1133,14 +1140,26 @@ static void pick_best(TuneResult& res) {
             if ((t.cfg.kind == PUSH_LOCAL) == local) least = std::min(least, t.ms);
         const TuneEntry* pick = nullptr;
         for (const TuneEntry& t : res.report) {
-            if ((t.cfg.kind == PUSH_LOCAL) != local || t.ms > least * (1.0f + kTuneTie)) continue;
+            if ((t.cfg.kind == PUSH_LOCAL) != local) continue;
+            if (t.cfg.kind == PUSH_REG && t.cfg.param == 8 && t.cfg.lpr == 32 && t.ms <= least * (1.0f + kTuneDefault)) return &t;
+            if (t.ms > least * (1.0f + kTuneTie)) continue;
             if (!pick || (weigh && whole(&t) < whole(pick))) pick = &t;
         }
         return pick;
     };
     const TuneEntry* pick = fastest(false);
     const TuneEntry* local = res.dense ? fastest(true) : nullptr;       // no step reached the threshold: only scatters
-    if (local && whole(local) + kWindowStepMs < whole(pick)) pick = local;
+    if (local) {
+        double scatter = whole(pick);
+        if (n_nets > 1) {
+            for (const TuneEntry& t : res.report)
+                if (t.cfg.kind != PUSH_LOCAL) scatter = std::min(scatter, whole(&t));
+            scatter *= 1.0 - kTuneBatch;
+        } else {
+            scatter *= 1.0 + kTuneTie;      // one network bursts as a whole: a tie goes to the windows
+        }
+        if (whole(local) + kWindowStepMs < scatter) pick = local;
+    }
     res.best = pick->cfg;
     res.best_ms = pick->ms;
 }
@@ -1169,7 +1188,7 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         if (res.observed >= res.observe + kTuneGiveUp) {
             // settle: the best of the samples so far, or the default variant
             res.tuned = true;
-            pick_best(res);
+            pick_best(res, b.n_nets);
         }
         return DTB_OK;
     }
@@ -1275,7 +1294,7 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
     // a common step too, where some steps reach the windows' threshold and some do not
     if (res.samples < res.want || (windows && res.quiet.empty() && res.dense && res.dense < res.observed)) return DTB_OK;
     res.tuned = true;
-    pick_best(res);
+    pick_best(res, b.n_nets);
     return DTB_OK;
 }
 

@@ -238,8 +238,8 @@ int32_t dtb_info(void* engine, dtb_engine_info* info);
  * every step for 50 steps, then times every variant on the live spike lists of
  * four steps with at least half the peak count seen (and 0.2 % of the neurons),
  * 47 or more steps apart, and of one step with the mean load of those in which
- * window forms scatter.  It keeps the variant with the smallest mean over the four,
- * a window form only if it also wins when both kinds of step are weighed by how
+ * window forms scatter.  It keeps the variant with the smallest mean over the four
+ * (kind 0 param 8 when that is within 4 % of it), a window form only if it also wins when both kinds of step are weighed by how
  * often they were read; it gives up (keeping the best so far, or the default)
  * after 400 reads of quiet steps.  The default, also after kind < 0 until a variant
  * is chosen, is kind 0 with param 8, or 1008 where rows hold fewer than 24 synapses
