@@ -1247,8 +1247,9 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         // Replays go in rounds, so that a slow moment (clocks rising after the read's wait) falls on
         // one replay of several variants, not on all of one's.  A busy step counts with the least of
         // three; a common step is a few of the events' 2 us ticks long and counts with the mean of
-        // the lower two thirds of nine.
-        const int reps = common ? 9 : 3;
+        // the lower two thirds of nine (of five in a batch, which serves requests meanwhile and
+        // decides by more than such a tick).
+        const int reps = !common ? 3 : b.n_nets > 1 ? 5 : 9;
         std::vector<std::vector<float>> ms_of(step.size());
         for (int rep = 0; rep < reps; ++rep) {
             for (size_t k = 0; k < step.size(); ++k) {
@@ -1269,7 +1270,7 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
         for (size_t k = 0; k < step.size(); ++k) {
             std::sort(ms_of[k].begin(), ms_of[k].end());
             step[k].ms = ms_of[k][0];
-            if (common) res.quiet.push_back({step[k].cfg, std::accumulate(ms_of[k].begin(), ms_of[k].begin() + 6, 0.0f) / 6.0f});
+            if (common) res.quiet.push_back({step[k].cfg, std::accumulate(ms_of[k].begin(), ms_of[k].begin() + reps * 2 / 3, 0.0f) / static_cast<float>(reps * 2 / 3)});
         }
         DTB_CU(reset_units());
         return DTB_OK;
