@@ -107,35 +107,38 @@ compact_write_kernel(const uint32_t* __restrict__ bits, uint32_t n, const uint32
     }
 }
 
-// The whole compaction of a small bitmap in one launch without scratch: CTA b writes the
-// spikes of words [1024 b, 1024 b + 1024) and counts the words before them itself.  The
-// re-read prefixes come from L2 (48 MB over the grid at 5M neurons, about 3 us) and cost less
-// than two more launches and a scratch buffer.  V4: the bitmap starts on a 16-byte boundary.
-template <bool V4>
-__global__ void __launch_bounds__(kDirectWords)
-compact_direct_kernel(const uint32_t* __restrict__ bits, uint32_t n, uint32_t* __restrict__ idx, uint32_t* __restrict__ count) {
-    __shared__ uint32_t s_own[kDirectWords / 32], s_before[kDirectWords / 32];
-    const uint32_t n_words = (n + 31) / 32, first = blockIdx.x * kDirectWords;
+// The whole compaction of a small bitmap in one launch without scratch: CTA b writes the spikes of
+// its `per` words (W consecutive words a thread; a multiple of 4) and counts the words before them
+// itself.  The re-read prefixes come from L2 and cost less than two more launches and a scratch
+// buffer.  V4: the bitmap starts on a 16-byte boundary.
+template <bool V4, int W>
+__global__ void __launch_bounds__(kDirectThreads)
+compact_direct_kernel(const uint32_t* __restrict__ bits, uint32_t n, uint32_t per, uint32_t* __restrict__ idx,
+                      uint32_t* __restrict__ count) {
+    __shared__ uint32_t s_own[kDirectThreads / 32], s_before[kDirectThreads / 32];
+    const uint32_t n_words = (n + 31) / 32, first = blockIdx.x * per, end = min(first + per, n_words);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t w = first + threadIdx.x;
-    uint32_t x = 0;
-    if (w < n_words) {
-        x = __ldg(bits + w);
-        if (w == n_words - 1 && (n & 31u)) x &= (1u << (n & 31u)) - 1u;
+    const uint32_t w0 = first + threadIdx.x * W;
+    uint32_t x[W];
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        x[k] = w0 + k < end ? __ldg(bits + w0 + k) : 0u;
+        if (w0 + k == n_words - 1 && (n & 31u)) x[k] &= (1u << (n & 31u)) - 1u;
+        c += __popc(x[k]);
     }
     uint32_t before = 0;
     if constexpr (V4) {
         const uint4* b4 = reinterpret_cast<const uint4*>(bits);
 #pragma unroll 8
-        for (uint32_t q = threadIdx.x; q < first / 4; q += kDirectWords) {
+        for (uint32_t q = threadIdx.x; q < first / 4; q += kDirectThreads) {
             const uint4 y = __ldg(b4 + q);
             before += __popc(y.x) + __popc(y.y) + __popc(y.z) + __popc(y.w);
         }
     } else {
 #pragma unroll 8
-        for (uint32_t q = threadIdx.x; q < first; q += kDirectWords) before += __popc(__ldg(bits + q));
+        for (uint32_t q = threadIdx.x; q < first; q += kDirectThreads) before += __popc(__ldg(bits + q));
     }
-    const uint32_t c = __popc(x);
     uint32_t incl = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -151,19 +154,29 @@ compact_direct_kernel(const uint32_t* __restrict__ bits, uint32_t n, uint32_t* _
     // spikes before this warp: all of the prefix, and the CTA's earlier warps
     const uint32_t mine = s_before[lane] + (lane < warp ? s_own[lane] : 0u);
     uint32_t pos = __reduce_add_sync(0xffffffffu, mine) + incl - c;
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kDirectWords - 1) *count = pos + c;
-    while (x) {
-        idx[pos++] = w * 32 + static_cast<uint32_t>(__ffs(x) - 1);
-        x &= x - 1;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kDirectThreads - 1) *count = pos + c;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        while (x[k]) {
+            idx[pos++] = (w0 + k) * 32 + static_cast<uint32_t>(__ffs(x[k]) - 1);
+            x[k] &= x[k] - 1;
+        }
     }
 }
 
-cudaError_t compact_direct(const uint32_t* bits, uint32_t n, uint32_t* idx, uint32_t* count, cudaStream_t s) {
-    const uint32_t blocks = ((n + 31) / 32 + kDirectWords - 1) / kDirectWords;
+template <int W>
+static void compact_direct_w(const uint32_t* bits, uint32_t n, uint32_t per, uint32_t* idx, uint32_t* count, cudaStream_t s) {
+    const uint32_t blocks = ((n + 31) / 32 + per - 1) / per;
     if ((reinterpret_cast<uintptr_t>(bits) & 15u) == 0)
-        compact_direct_kernel<true><<<blocks, kDirectWords, 0, s>>>(bits, n, idx, count);
+        compact_direct_kernel<true, W><<<blocks, kDirectThreads, 0, s>>>(bits, n, per, idx, count);
     else
-        compact_direct_kernel<false><<<blocks, kDirectWords, 0, s>>>(bits, n, idx, count);
+        compact_direct_kernel<false, W><<<blocks, kDirectThreads, 0, s>>>(bits, n, per, idx, count);
+}
+
+cudaError_t compact_direct(const uint32_t* bits, uint32_t n, uint32_t* idx, uint32_t* count, cudaStream_t s) {
+    const uint32_t even = ((n + 31) / 32 + kDirectCtas - 1) / kDirectCtas;   // words a CTA with one CTA an SM
+    if (even <= kDirectThreads) compact_direct_w<1>(bits, n, kDirectThreads, idx, count, s);
+    else compact_direct_w<2>(bits, n, (even + 3) / 4 * 4, idx, count, s);
     return cudaGetLastError();
 }
 

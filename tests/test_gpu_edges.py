@@ -16,6 +16,7 @@ DIRECT = 8 << 20           # its largest bitmap
 
 
 @pytest.mark.parametrize("n,offset", [(CTA - 1, 0), (CTA, 0), (CTA + 1, 0), (3 * CTA + 17, 1), (40 * CTA + 5, 3),
+                                      (148 * CTA, 0), (148 * CTA + 1, 0), (148 * CTA + 33, 3), (6_500_000, 0), (6_500_001, 1),
                                       (DIRECT, 0), (DIRECT + 1, 0), (DIRECT - 31, 2)])
 def test_compaction_edges(gpu, n, offset):
     import torch
