@@ -1635,7 +1635,8 @@ lif_pull_kernel(const NetView* __restrict__ nets, const uint32_t* __restrict__ t
 // kPullSmemNeurons neurons fits its bitmap beside one persistent CTA per SM, so an edge costs
 // one shared-memory word instead of a dependent access to L1 or L2 -- the chain of an in-edge
 // id and its bitmap word bounded the kernel above at a quarter of the copy bandwidth.  Warps
-// take groups of 32 neurons, strided over the grid; 16 edges in flight per lane.
+// take groups of 32 neurons, strided over the grid; 16 edges in flight per lane.  For rows of
+// kPullSmemDegree edges and more (both sides measured there).
 constexpr int kPullSmemThreads = 768;
 constexpr uint32_t kPullSmemNeurons = 1600u * 1024u;        // 200 KiB of bitmap
 
@@ -1663,6 +1664,8 @@ lif_pull_smem_kernel(const NetView* __restrict__ nets, uint32_t flags, int prop_
     uint32_t err = 0;
     const PullStep ps = pull_step(nv, flags, prop_mode, err);
     stage_bitmap(s_bits, (ps.n & 1ull) ? nv.bits0 : nv.bits1, nv.n_words);
+    // the first kStatSlots populations; the others go to global sums warp by warp (slots for 1,024
+    // populations measured the same with 20 to 2,000 of them)
     const StatAcc sa{s_cnt, s_vs, 0u};
     const uint32_t warps = gridDim.x * (kPullSmemThreads / 32);
     for (uint32_t g = warp * gridDim.x + blockIdx.x; g < nv.n_words; g += warps)

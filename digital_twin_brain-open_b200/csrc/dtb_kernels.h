@@ -27,7 +27,8 @@ constexpr uint32_t kUnitsPerSm = 4;
 // 6.0 to 6.5 ps per event; the windows cost about 3.5 ps and 40 to 60 us of preparation, unit
 // start-up and uneven ends.  Measured, windows against scatter: 86 / 41 us at 6.0e6 events (250k
 // neurons, BF16, fixed), 84 / 82 us at 1.3e7, 110 / 118 us at 1.9e7 (200k, FP32, float),
-// 158 / 217 us at 3.2e7.
+// 158 / 217 us at 3.2e7.  All four are single networks; a batch uses the same line, and whether its
+// windows, spread over the members, pay over a run is the tuner's to find.
 constexpr uint64_t kDenseEvents = 16000000;
 // Networks whose every synapse together stays below kDenseEvents never take windows, and the
 // register-staged forms are within 5 % of each other on them (8.1 to 8.6 us on the 10,000-neuron
