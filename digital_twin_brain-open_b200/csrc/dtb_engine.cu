@@ -1292,8 +1292,8 @@ int tune_push_views(const LaunchBatch& b, const std::vector<NetView>& views, int
                 res.report[k].ms += (step[k].ms - res.report[k].ms) / static_cast<float>(res.samples);
         }
     }
-    // a common step too, where some steps reach the windows' threshold and some do not
-    if (res.samples < res.want || (windows && res.quiet.empty() && res.dense && res.dense < res.observed)) return DTB_OK;
+    // a common step too, where most steps stay below the windows' threshold and some do not
+    if (res.samples < res.want || (windows && res.quiet.empty() && res.dense && 2 * res.dense < res.observed)) return DTB_OK;
     res.tuned = true;
     pick_best(res, b.n_nets);
     return DTB_OK;
