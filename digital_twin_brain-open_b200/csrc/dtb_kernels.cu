@@ -764,6 +764,29 @@ __device__ __forceinline__ void push_span(const uint32_t* col, const void* wts, 
     }
 }
 
+// All synapses of a row, from CSR slot beg up to end.  64-bit positions, unlike push_span: the
+// compiler folds their constant distances into the loads.
+template <int ACC, int WT, int U, int LPR>
+__device__ __forceinline__ void push_row(const uint32_t* col, const void* wts, const PushDst& d, unsigned long long beg,
+                                         unsigned long long end, uint32_t lane, unsigned long long keep) {
+    const unsigned long long len = end - beg;
+    for (unsigned long long x = lane; x < len; x += static_cast<unsigned long long>(LPR) * U) {
+        uint32_t c[U];
+        float2 w[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const unsigned long long xq = x + static_cast<unsigned long long>(LPR) * q;
+            if (xq < len) {
+                c[q] = __ldcs(col + beg + xq);
+                w[q] = load_weight<WT>(wts, beg + xq);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (x + static_cast<unsigned long long>(LPR) * q < len) reduce_synapse<ACC>(d, c[q], w[q], keep);
+    }
+}
+
 // Whole rows of the spike list, LPR lanes per row: 32 (a warp per row) or 16 / 8 (2 / 4 rows
 // per warp, for short rows).  With fewer rows than groups of lanes, a row is cut into
 // interleaved parts of U x LPR synapses so that a quiet step (a few dozen rows, most of the
@@ -795,9 +818,13 @@ __device__ __forceinline__ void push_rows(const NetView* __restrict__ nets, cons
             d = push_dst<ACC>(nets[k]);
         }
         const uint32_t j = v - vb;
-        const unsigned long long beg = __ldg(ptr + j);
-        const uint32_t len = static_cast<uint32_t>(__ldg(ptr + j + 1) - beg);
-        push_span<ACC, WT, U, LPR, false>(col, wts, d, beg, len, 0ull, len, lane + part * (LPR * U), parts * (LPR * U), keep);
+        const unsigned long long beg = __ldg(ptr + j), end = __ldg(ptr + j + 1);
+        if constexpr (CUT) {
+            const uint32_t len = static_cast<uint32_t>(end - beg);
+            push_span<ACC, WT, U, LPR, false>(col, wts, d, beg, len, 0ull, len, lane + part * (LPR * U), parts * (LPR * U), keep);
+        } else {
+            push_row<ACC, WT, U, LPR>(col, wts, d, beg, end, lane, keep);
+        }
     }
 }
 
